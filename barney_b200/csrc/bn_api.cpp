@@ -172,6 +172,92 @@ static IsoDD isoDD(const IsoSurface &g, const float2 *ranges, const int mcDims[3
 }
 
 // ---------------------------------------------------------------------------
+// pixels whose rays cannot meet the volume
+// ---------------------------------------------------------------------------
+// Edges of the projection of the field's bounds, in pixels, for
+// FrameDD::cull: a pixel beyond an edge by more than the error margin sends
+// no ray that passes the box test of traceBegin.  The projection of a box in
+// front of the camera is the convex hull of its corners' projections; without
+// that (a corner beside or behind the camera, a cut plane that moves ray
+// origins, non-finite input) no pixel is ruled out.
+//
+// The margin covers what separates the kernels' binary32 rays from the exact
+// ones: one pixel, plus an angle of 1e-5 (the zero fix-up of a direction's
+// components moves it by at most 1e-6 each; rounding of the direction and of
+// the box test's slab distances is below 2e-6).
+static void cullEdges(const VolumeDD &v, FrameDD &fr) {
+  for (auto &e : fr.cull) e = make_float3(0.f, 0.f, 0.f);
+  if (fr.cutPlane.w > -1e28f) return;
+  const double d0[3] = {fr.dir00.x, fr.dir00.y, fr.dir00.z}, du[3] = {fr.dirdu.x, fr.dirdu.y, fr.dirdu.z},
+               dv[3] = {fr.dirdv.x, fr.dirdv.y, fr.dirdv.z}, o[3] = {fr.lens00.x, fr.lens00.y, fr.lens00.z};
+  // rows of the inverse of [d0 du dv]
+  auto crs = [](const double *a, const double *b, double *r) {
+    r[0] = a[1] * b[2] - a[2] * b[1];
+    r[1] = a[2] * b[0] - a[0] * b[2];
+    r[2] = a[0] * b[1] - a[1] * b[0];
+  };
+  auto dt = [](const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
+  double r0[3], ru[3], rv[3];
+  crs(du, dv, r0);
+  crs(dv, d0, ru);
+  crs(d0, du, rv);
+  const double det = dt(d0, r0);
+  if (!(std::fabs(det) > 1e-12) || !std::isfinite(det)) return;
+  for (int a = 0; a < 3; a++) { r0[a] /= det; ru[a] /= det; rv[a] /= det; }
+  const double W = fr.width, H = fr.height, aspect = fr.aspect;
+  // the error of a ray in pixels: an angle of 1e-5 against the longest
+  // unnormalised direction of the image, through the inverse's rows
+  const double su = 0.5 * aspect, sv = 0.5;
+  const double len = std::sqrt(dt(d0, d0)) + su * std::sqrt(dt(du, du)) + sv * std::sqrt(dt(dv, dv));
+  const double n0 = std::sqrt(dt(r0, r0)), nu = std::sqrt(dt(ru, ru)), nv = std::sqrt(dt(rv, rv));
+  const double ex = 1e-5 * len * (nu + 2 * su * n0) / aspect * W, ey = 1e-5 * len * (nv + 2 * sv * n0) * H;
+  double px[8], py[8];
+  for (int c = 0; c < 8; c++) {
+    const double q[3] = {((c & 1) ? v.boundsHi.x : v.boundsLo.x) - o[0], ((c & 2) ? v.boundsHi.y : v.boundsLo.y) - o[1],
+                         ((c & 4) ? v.boundsHi.z : v.boundsLo.z) - o[2]};
+    const double depth = dt(r0, q);
+    // in front of the camera by a margin against the distance, so that the
+    // projection is well-conditioned
+    if (!(depth > 1e-3 * n0 * std::sqrt(dt(q, q))) || !(depth > 0.0)) return;
+    px[c] = (dt(ru, q) / depth / aspect + 0.5) * W;
+    py[c] = (dt(rv, q) / depth + 0.5) * H;
+    if (!std::isfinite(px[c]) || !std::isfinite(py[c]) || std::fabs(px[c]) > 1e7 || std::fabs(py[c]) > 1e7) return;
+  }
+  // convex hull by gift wrapping from the leftmost corner; an edge of the hull
+  // keeps every corner on its inner side
+  int start = 0;
+  for (int c = 1; c < 8; c++)
+    if (px[c] < px[start] || (px[c] == px[start] && py[c] < py[start])) start = c;
+  int cur = start, edges = 0;
+  do {
+    int next = -1;
+    for (int c = 0; c < 8; c++) {
+      if (px[c] == px[cur] && py[c] == py[cur]) continue;
+      if (next < 0) { next = c; continue; }
+      const double t = (px[next] - px[cur]) * (py[c] - py[cur]) - (py[next] - py[cur]) * (px[c] - px[cur]);
+      const auto d2 = [&](int k) { return (px[k] - px[cur]) * (px[k] - px[cur]) + (py[k] - py[cur]) * (py[k] - py[cur]); };
+      if (t < 0 || (t == 0 && d2(c) > d2(next))) next = c;
+    }
+    if (next < 0) return;  // all corners project to one point
+    // outward normal of the edge cur -> next (corners on its left)
+    double a = py[next] - py[cur], b = -(px[next] - px[cur]);
+    const double l = std::sqrt(a * a + b * b);
+    a /= l;
+    b /= l;
+    double off = -1e300;  // the farthest corner along the normal
+    for (int c = 0; c < 8; c++) off = std::max(off, a * px[c] + b * py[c]);
+    // every point of the pixel's square lies beyond the edge by the margin:
+    // half the square and one pixel along the normal, the ray's error, and
+    // the binary32 rounding of the kernel's test
+    const double margin = 1.5 * (std::fabs(a) + std::fabs(b)) + std::fabs(a) * ex + std::fabs(b) * ey +
+                          1e-6 * (W + H + std::fabs(off));
+    if (edges < kCullEdges) fr.cull[edges] = make_float3((float)a, (float)b, (float)(-off - margin));
+    edges++;
+    cur = next;
+  } while (cur != start && edges < 16);
+}
+
+// ---------------------------------------------------------------------------
 // render (Context::renderTiles, Context.cpp:139-182, + finalizeFrame)
 // ---------------------------------------------------------------------------
 // The device job of one (renderer, model, camera, frame buffer) tuple,
@@ -247,6 +333,7 @@ JobDD buildJob(Context *ctx, Renderer &r, Model &m, Camera &cam, FrameBuffer &fb
   fr.spp = p.pathsPerPixel;
   fr.color = fb.color.ptr;
   fr.colorFormat = fb.colorFormat;
+  cullEdges(v, fr);
   return job;
 }
 
@@ -312,8 +399,9 @@ static cudaError_t launchRenderJob(Context *ctx, const JobDD &job, cudaStream_t 
     return job.fr.fastMath ? fastmath::launchRenderRegrouped(job.v, job.fr, ctx->dCounters, s)
                            : launchRenderRegrouped(job.v, job.fr, ctx->dCounters, s);
   if (job.fr.fastMath && plain)
-    return fastmath::launchRender(job.v, job.fr, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched);
-  return launchRender(job.v, job.fr, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched);
+    return fastmath::launchRender(job.v, job.fr, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
+                                  ctx->ring);
+  return launchRender(job.v, job.fr, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched, ctx->ring);
 }
 
 static void render(Context *ctx, Renderer &r, Model &m, Camera &cam, FrameBuffer &fb) {
@@ -439,19 +527,16 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
        "chunk table");
     ck(cudaMemsetAsync(ctx->dCounters, 0, sizeof(LaunchCounters), s), "counter reset");
     if (timed) ck(cudaEventRecord(ctx->ev[0], s), "event");
-    const int compMode = compJobs == 0 ? 0 : compJobs == n ? 2 : 1;
     if (!ctx->useGraphs && extended == 0 && n <= kParamJobs)  // the jobs as one kernel parameter
       ck((fast ? fastmath::launchRenderBatchParams : launchRenderBatchParams)(
              ctx->hostJobs, ctx->hostChunks, n, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
-             voxelType, compMode),
+             voxelType, ctx->ring),
          "batch render kernel");
     else
-    ck((fast ? fastmath::launchRenderBatch : launchRenderBatch)((const JobDD *)ctx->batchJobs.ptr,
-                                                                (const int *)ctx->batchChunks.ptr, n, ctx->dCounters,
-                                                                ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
-                                                                extended, voxelType,
-                                                                compJobs == 0 ? 0 : compJobs == n ? 2 : 1),
-       "batch render kernel");
+      ck((fast ? fastmath::launchRenderBatch : launchRenderBatch)(
+             (const JobDD *)ctx->batchJobs.ptr, (const int *)ctx->batchChunks.ptr, n, (int)chunks, ctx->dCounters,
+             ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched, extended, voxelType, compJobs > 0, ctx->ring),
+         "batch render kernel");
     if (timed) ck(cudaEventRecord(ctx->ev[1], s), "event");
     ck(launchResolveBatch((const JobDD *)ctx->batchJobs.ptr, (const int *)ctx->batchChunks.ptr, n, (int)chunks, s),
        "batch resolve kernel");

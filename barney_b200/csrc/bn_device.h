@@ -19,11 +19,16 @@ constexpr long long kMaxFramePixels = 0x7fffffffLL;  // pixels of one frame (32-
 constexpr int kPartTileChunks = 32;    // pixel-tile partition: 32 chunks of 32 pixels per tile
 constexpr int kRenderMaxThreads = 128;  // __launch_bounds__ of the render kernels:
 constexpr int kRenderMinBlocks = 7;     // plain: 7 x 128 threads per SM (at most 73 registers)
-constexpr int kRenderMinBlocksMixedComp = 6;  // plain, compensated sums tested per job (mixed batches):
-                                              // 6 x 128 (85; at 7 they spill up to 348 B)
 constexpr int kRenderMinBlocksExt = 5;  // extended (multi-scatter, principled): 5 x 128 (102)
 constexpr int kRenderMinBlocksIso = 4;  // extended with isosurfaces: 4 x 128 (128; with the warp-cooperative
                                         // iso scan 3 % faster than 5 x 128, which spilled up to 820 B)
+
+constexpr int kCullEdges = 6;           // a box projects to at most a hexagon
+// Streamed render loop: paths of a ring slot, slots of a warp's ring.
+constexpr int kStreamSlotPaths = 64;
+constexpr unsigned kStreamSlots = 16;
+constexpr int kStreamRing = kStreamSlotPaths * (int)kStreamSlots;  // ring entries (float4) of a warp
+constexpr int kStreamWarpsPerSM = 32;  // warps per SM a context holds rings for
 
 // Principled volume coefficients evaluated from the field value
 // (PrincipledVolumeParams::DD, PrincipledVolume.h:33-46).
@@ -98,6 +103,10 @@ struct FrameDD {
   int partRank, partCount;  // pixel-tile partition: render the tiles t with t % partCount == partRank
   float4 *accum;        // width*height, linear
   float4 *comp;         // width*height Neumaier compensation terms, or null (plain sums)
+  // edges of the volume bounds' projection in pixels: pixel (x, y) with
+  // a (x + .5) + b (y + .5) + c > 0 for some edge sends no ray that meets the
+  // bounds (bn_api.cpp cullEdges; all zero: no pixel is ruled out)
+  float3 cull[kCullEdges];
   int accumID0;         // accumID of the first wave of this launch
   int spp;              // waves in this launch
   void *color;          // resolved output (batch resolve only)
@@ -117,6 +126,8 @@ struct JobDD {
 // serves them together.
 struct SchedDD {
   int serviceBatch = 22;
+  int sampleBatch = 26;  // streamed loop: lanes no longer walking before the steps among them are sampled
+  int unitSplit = 0;  // streamed loop: log2 of the units a 32-pixel chunk is cut into (set by the launchers)
   int regrouped = 0;  // plain single-frame jobs: the regrouped kernel (launchRenderRegrouped) instead of renderLoop's
 };
 
@@ -127,6 +138,15 @@ struct LaunchCounters {
   unsigned int abort;       // host-set abort request
 };
 
+// Ring memory of the streamed render loop: kStreamRing float4 for each of
+// `warps` warps.  A launch uses it until it ends; launches that can run at the
+// same time need rings of their own (one per context, whose launches are
+// ordered by its stream).
+struct StreamRing {
+  float4 *ptr = nullptr;
+  int warps = 0;
+};
+
 // launchers (bn_kernels.cu).  Both majorant launchers also write the
 // occupancy bitmap of the new majorants, ceil(n/32) words; with majorants
 // null, launchBuildMacrocells writes the scalar ranges only.
@@ -135,27 +155,26 @@ cudaError_t launchBuildMacrocells(const VolumeDD &vol, float2 *ranges, float *ma
 cudaError_t launchMapMajorants(const VolumeDD &vol, const float2 *ranges, float *majorants, unsigned *occupied,
                                int roundUp, cudaStream_t s);
 cudaError_t launchRender(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, int blocksPerSM,
-                         int threadsPerBlock, cudaStream_t s, const SchedDD &sd = SchedDD());
+                         int threadsPerBlock, cudaStream_t s, const SchedDD &sd, const StreamRing &ring);
 // jobs / chunkStart: device arrays; chunkStart has numJobs+1 entries, the
-// prefix sum of each job's ceil(width*height/32) pixel chunks.
+// prefix sum of each job's ceil(width*height/32) pixel chunks, numChunks in all.
 // extended: 2 if some job has an isosurface and some job volume bounces
 // (fr.maxVolumeBounces > 0) or a principled volume, 3 if some job has an
 // isosurface and none has either, else 1 if some job has volume bounces, a
 // principled volume or exact-log free flight, else 0 (selects the kernel
 // instantiation that implements them); voxelType: the
 // VoxelType all jobs share (a kernel compiled for it) or -1 (mixed);
-// compensated: how many jobs carry compensation terms (fr.comp): 0 none,
-// 1 some, 2 all
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, LaunchCounters *counters,
-                              int blocksPerSM, int threadsPerBlock, cudaStream_t s, const SchedDD &sd = SchedDD(),
-                              int extended = 0, int voxelType = -1, int compensated = 1);
+// compensated (extended kernels): some job carries compensation terms (fr.comp)
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
+                              LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
+                              SchedDD sd, int extended, int voxelType, int compensated, const StreamRing &ring);
 // The same for at most kParamJobs plain jobs (extended 0) whose table and
 // chunk prefix are in host memory: passed as one kernel parameter.  Not for
 // stream capture (the parameter would be frozen into the graph).
-constexpr int kParamJobs = 32;
+constexpr int kParamJobs = 31;
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
                                     LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
-                                    const SchedDD &sd, int voxelType, int compensated);
+                                    SchedDD sd, int voxelType, const StreamRing &ring);
 cudaError_t launchResolve(const float4 *accum, int numPixels, int accumID, int fmt, void *out, cudaStream_t s,
                           const float4 *comp = nullptr);
 // resolves every job of a batch table into its fr.color after its waves
@@ -189,13 +208,13 @@ cudaError_t launchSampleProbe(const VolumeDD &vol, const float3 *P, int n, float
 // needs an extended kernel returns cudaErrorInvalidValue.
 namespace fastmath {
 cudaError_t launchRender(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, int blocksPerSM,
-                         int threadsPerBlock, cudaStream_t s, const SchedDD &sd = SchedDD());
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, LaunchCounters *counters,
-                              int blocksPerSM, int threadsPerBlock, cudaStream_t s, const SchedDD &sd = SchedDD(),
-                              int extended = 0, int voxelType = -1, int compensated = 1);
+                         int threadsPerBlock, cudaStream_t s, const SchedDD &sd, const StreamRing &ring);
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
+                              LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
+                              SchedDD sd, int extended, int voxelType, int compensated, const StreamRing &ring);
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
                                     LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
-                                    const SchedDD &sd, int voxelType, int compensated);
+                                    SchedDD sd, int voxelType, const StreamRing &ring);
 cudaError_t launchSampleProbe(const VolumeDD &vol, const float3 *P, int n, float *scalar, float4 *rgba, cudaStream_t s);
 cudaError_t launchRenderRegrouped(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, cudaStream_t s);
 long long readBoundsViolationsHere();  // bounds-checked build only

@@ -3,8 +3,8 @@
 //   mcBuildKernel      macrocell scalar ranges + majorants (StructuredData.cu:31-96,
 //                      MCGrid.cu:97-141), fused
 //   mcMapKernel        majorant re-map after a transfer-function change (mapMCs)
-//   renderKernel       persistent megakernel: ray generation (generateRays.cu:43-244),
-//                      box test + 3D-DDA over the macrocell grid (MCAccelerator.h:552-689,
+//   streamKernel,      persistent megakernels: ray generation (generateRays.cu:43-244),
+//   renderKernel       box test + 3D-DDA over the macrocell grid (MCAccelerator.h:552-689,
 //                      DDA.h:61-201), Woodcock tracking with software trilinear sampling
 //                      and TF lookup (Volume.h:62-203, StructuredData.h:101-112,
 //                      rtcore/cpu/Texture.cpp:324-416, TransferFunction.h:68-87),
@@ -17,12 +17,11 @@
 // expression is evaluated exactly as the reference source writes it; the
 // results are bit-identical to the FP32 CPU restatement in oracle/.
 //
-// Work decomposition: one warp owns an 8x4 pixel tile for all waves of the
-// launch; each lane owns one pixel and accumulates it in registers in wave
-// order (the order the reference's per-generation launches add in).  Warps
-// fetch tiles from a global counter.  Each loop iteration performs at most
-// one Woodcock step, so lanes on different rays, waves or generations keep
-// executing the sampling code together.
+// Work decomposition: plain jobs run streamLoop, where a lane traces any path
+// of its warp's pixels and the paths' outcomes are added up in wave order (the
+// order the reference's per-generation launches add in); extended jobs run
+// renderLoop, where each lane owns a pixel for all waves of the launch.  Warps
+// fetch pixels from a global counter.
 #include "bn_device.h"
 
 #include <cuda_fp16.h>
@@ -901,6 +900,7 @@ enum LanePhase : int {
   LP_WOODCOCK = 3,  // inside a Woodcock range
   LP_HIT = 4,       // collision found, waiting to be shaded
   LP_ENDED = 5,     // ray left the grid (primary: background; shadow: reached the light)
+  LP_SAMPLE = 7,    // streamed loop: a Woodcock step that may end inside its range, waiting for its sample
   LP_BEGIN = 6      // a new primary or shadow ray (ts.org, ts.dir, ts.rayTMax) needs its set-up
 };
 
@@ -1084,6 +1084,115 @@ DEV void isoNormalSamples(const JobDD *jobs, int job, const VolumeDD &v, float3 
     }
   }
   __syncwarp();
+}
+
+// Primary ray of pixel (ix, iy) in wave accumID (generateRays.cu:71-243):
+// origin, direction, tMax and the ray's RNG seed.
+DEV void primaryRay(const FrameDD &fr, int ix, int iy, int accumID, float3 &o, float3 &d, float &tMax,
+                    uint64_t &raySeed) {
+  const int W = fr.width, H = fr.height;
+  // 32-bit wrap-around arithmetic, as the reference's ints do on the GPU
+  const unsigned uAcc = (unsigned)accumID;
+  uint64_t rnd = rngSeed2((unsigned)ix + (unsigned)W * uAcc, (unsigned)iy + (unsigned)H * uAcc);
+  raySeed = rngSeed2((unsigned)ix + uAcc * (unsigned)W, (uint32_t)iy);
+  const float pixel_u = (accumID == 0) ? .5f : rngFloat(rnd);
+  const float pixel_v = (accumID == 0) ? .5f : rngFloat(rnd);
+  const float image_u = ((ix + pixel_u) / float(W));
+  const float image_v = ((iy + pixel_v) / float(H));
+  const float aspect = fr.aspect;  // W / float(H), formed on the host
+  const float su = 1.f * aspect * (image_u - .5f), sv = 1.f * (image_v - .5f);
+  d = f3(fr.dir00.x + su * fr.dirdu.x + sv * fr.dirdv.x, fr.dir00.y + su * fr.dirdu.y + sv * fr.dirdv.y,
+         fr.dir00.z + su * fr.dirdu.z + sv * fr.dirdv.z);
+  d = normalize3(d);
+  o = fr.lens00;
+  tMax = 1e30f;
+  if (fr.cutPlane.w > -1e28f) {
+    const float3 N = f3(fr.cutPlane.x, fr.cutPlane.y, fr.cutPlane.z);
+    const float dist_org = dot3(N, o) + fr.cutPlane.w;
+    const float denom = dot3(N, d);
+    if (dist_org >= 0.f) {
+      if (denom < 0.f) tMax = fmin_(tMax, -dist_org / denom);
+    } else {
+      if (denom > 0.f) {
+        const float te = -dist_org / denom;
+        o = f3(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
+      } else tMax = 0.f;
+    }
+  }
+}
+
+// The colour a primary ray of image row iy adds when it leaves the volume
+// (generateRays.cu:217-227).
+DEV float4 missColor(const FrameDD &fr, int iy) {
+  if (fr.bgColor.w >= 0.f) return fr.bgColor;
+  const float t = (iy + .5f) / float(fr.height);
+  return make_float4((1.0f - t) * 0.9f + t * 0.15f, (1.0f - t) * 0.9f + t * 0.25f, (1.0f - t) * 0.9f + t * .8f,
+                     (1.0f - t) * 1.f + t * 1.f);
+}
+
+// Pixel w of a frame in chunk order: 4-row bands, column-major inside a band
+// (8x4 tiles per 32 pixels).
+DEV void chunkPixel(const FrameDD &fr, int w, int &ix, int &iy) {
+  const int W = fr.width, H = fr.height;
+  const int band = w / (4 * W);
+  const int rows = min(4, H - 4 * band);
+  const int within = w - band * 4 * W;
+  ix = within / rows;
+  iy = 4 * band + within % rows;
+}
+
+// bounce() at a primary ray's volume collision (shadeRays.cu:608-746): samples
+// a light and forms the shadow ray (origin, direction, tMax; raySeed advanced
+// to its seed) and the fragment it adds if it reaches the light.  dir: the
+// ray's direction before the zero fix-up; tint: the TF colour at the hit.
+// Returns false if no shadow ray goes out.
+DEV bool shadeVolumeHit(const VolumeDD &v, const FrameDD &fr, float3 P, float tHit, float3 dir, float3 tint,
+                        float clampMax, uint64_t &raySeed, float3 &sOrg, float3 &sDir, float &sTMax, float3 &frag) {
+  uint64_t random = rngDerive(raySeed, (uint64_t)__float_as_uint(tHit));
+  const float3 won = normalize3(dir);
+  const float3 woN = f3(-won.x, -won.y, -won.z);  // dg.wo
+  const float offsetEpsilon = fmax_(1e-4f, 1e-6f * fmax_(fmax_(fabsf(P.x), fabsf(P.y)), fabsf(P.z)));
+  LightSample ls;
+  bool needsMIS, isDir;
+  if (!sampleLights(fr, random, ls, needsMIS, isDir)) return false;
+  float3 alb;
+  float fpdf;
+  if (v.phase == PHASE_SIMPLE) {
+    alb = f3(.7f * tint.x, .7f * tint.y, .7f * tint.z);
+    fpdf = kOneOverFourPi;
+  } else {
+    const float a = v.scatteringAlbedo;
+    alb = f3(a * tint.x, a * tint.y, a * tint.z);
+    // HGPhase::pdf (Phase.h:51-58) is 1/4pi for |g| < 1e-3 whatever the
+    // angle: the directions are normalised only when it is not
+    if (fabsf(v.anisotropy) < 1e-3f) {
+      fpdf = kOneOverFourPi;
+    } else {
+      const float3 wi_in = normalize3(f3(-woN.x, -woN.y, -woN.z));
+      fpdf = hgPhase(v.anisotropy, dot3(wi_in, normalize3(ls.dir)));
+    }
+  }
+  float3 fv = f3(fpdf * alb.x, fpdf * alb.y, fpdf * alb.z);
+  if (!(fpdf > 0.f) || fmax_(fmax_(fv.x, fv.y), fv.z) < 1e-4f) return false;
+  fv = f3(fmin_(fv.x, 13.f), fmin_(fv.y, 13.f), fmin_(fv.z, 13.f));
+  const float ip = isinf(ls.pdf) ? 1.f : (1.f / ls.pdf);
+  const float3 tp = f3(1.f * ip * fv.x * ls.radiance.x * 1.f, 1.f * ip * fv.y * ls.radiance.y * 1.f,
+                       1.f * ip * fv.z * ls.radiance.z * 1.f);
+  float misWeight = 1.f;
+  if (!isDir && needsMIS) {
+    // the phase pdf of the light sample's direction is fpdf
+    // (the same expression: 1/4pi, or hgPhase of the same vectors)
+    misWeight = kOneOverFourPi / (kOneOverFourPi + fpdf + 1e-10f);
+    if (misWeight < 1e-5f) return false;
+  }
+  sTMax = kInf * (1.f - 2.f * offsetEpsilon);
+  if (!(sTMax > 0.f)) return false;
+  frag = f3(fmin_(misWeight * roundHalf(tp.x), clampMax), fmin_(misWeight * roundHalf(tp.y), clampMax),
+            fmin_(misWeight * roundHalf(tp.z), clampMax));
+  // makeShadowRay (Ray.h:147-157)
+  sOrg = f3(P.x + offsetEpsilon * woN.x, P.y + offsetEpsilon * woN.y, P.z + offsetEpsilon * woN.z);
+  sDir = ls.dir;
+  return true;
 }
 
 // The render loop shared by the single-frame kernel (one job, read from a
@@ -1536,36 +1645,9 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       //    (generateRays.cu:71-243)
       // ------------------------------------------------------------------
       if (phase == LP_NEWSAMPLE) {
-        const int W = fr.width, H = fr.height;
-        const int accumID = fr.accumID0 + k;
-        // 32-bit wrap-around arithmetic, as the reference's ints do on the GPU
-        const unsigned uAcc = (unsigned)accumID;
-        uint64_t rnd = rngSeed2((unsigned)ix + (unsigned)W * uAcc, (unsigned)iy + (unsigned)H * uAcc);
-        raySeed = rngSeed2((unsigned)ix + uAcc * (unsigned)W, (uint32_t)iy);
-        const float pixel_u = (accumID == 0) ? .5f : rngFloat(rnd);
-        const float pixel_v = (accumID == 0) ? .5f : rngFloat(rnd);
-        const float image_u = ((ix + pixel_u) / float(W));
-        const float image_v = ((iy + pixel_v) / float(H));
-        const float aspect = fr.aspect;  // W / float(H), formed on the host
-        const float su = 1.f * aspect * (image_u - .5f), sv = 1.f * (image_v - .5f);
-        float3 d = f3(fr.dir00.x + su * fr.dirdu.x + sv * fr.dirdv.x, fr.dir00.y + su * fr.dirdu.y + sv * fr.dirdv.y,
-                      fr.dir00.z + su * fr.dirdu.z + sv * fr.dirdv.z);
-        d = normalize3(d);
-        float3 o = fr.lens00;
-        float tMax = 1e30f;
-        if (fr.cutPlane.w > -1e28f) {
-          const float3 N = f3(fr.cutPlane.x, fr.cutPlane.y, fr.cutPlane.z);
-          const float dist_org = dot3(N, o) + fr.cutPlane.w;
-          const float denom = dot3(N, d);
-          if (dist_org >= 0.f) {
-            if (denom < 0.f) tMax = fmin_(tMax, -dist_org / denom);
-          } else {
-            if (denom > 0.f) {
-              const float te = -dist_org / denom;
-              o = f3(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
-            } else tMax = 0.f;
-          }
-        }
+        float3 o, d;
+        float tMax;
+        primaryRay(fr, ix, iy, fr.accumID0 + k, o, d, tMax, raySeed);
         if (EXT) primDir = d;
         shadowRay = false;
         if (EXT) {
@@ -1727,11 +1809,11 @@ __host__ __device__ inline int partitionChunks(int numChunks, int rank, int coun
   return (mine - 1) * kPartTileChunks + min(kPartTileChunks, numChunks - last * kPartTileChunks);
 }
 
+#ifndef BNB_FAST_MATH
 template <int T, int LOG, int EXT, int CMP>
-__global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2     ? kRenderMinBlocksIso
-                                                     : EXT        ? kRenderMinBlocksExt
-                                                     : CMP == 1   ? kRenderMinBlocksMixedComp
-                                                                  : kRenderMinBlocks)
+__global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2 ? kRenderMinBlocksIso
+                                                     : EXT    ? kRenderMinBlocksExt
+                                                              : kRenderMinBlocks)
     renderKernel(const __grid_constant__ JobDD job, const __grid_constant__ SchedDD sd, LaunchCounters *ctr) {
   extern __shared__ float4 sTF[];
   __shared__ float u8lut[256];
@@ -1743,6 +1825,607 @@ __global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2     ? kRenderMinBl
   if (job.fr.partCount > 1) numChunks = partitionChunks(numChunks, job.fr.partRank, job.fr.partCount);
   renderLoop<T, false, LOG, EXT, CMP>(&job, nullptr, 1, numChunks, sd, ctr, sTF, u8lut,
                                       EXT >= 2 ? sIsoBuf + (threadIdx.x >> 5) * kIsoBufPerWarp : nullptr);
+}
+#endif  // !BNB_FAST_MATH
+
+// ---------------------------------------------------------------------------
+// Streamed render loop (plain jobs)
+// ---------------------------------------------------------------------------
+// A lane traces one path at a time, any path of the warp's work: a path is
+// (pixel, wave), and a finished path writes its outcome -- missed the volume,
+// its light was occluded, or the fragment its shadow ray adds -- to the warp's
+// ring in global memory (L2).  The ring is cut into slots of up to
+// kStreamSlotPaths paths of one unit (up to 32 neighbouring pixels, all waves);
+// when every path of the oldest slot is done, its pixels add their outcomes in
+// wave order, which is the order the reference's per-generation launches add
+// in, so sums are bit-identical to a lane that owns its pixel.
+//
+// A service pass gives all waiting lanes the same kind of work: either new
+// primary rays, or collisions to shade (those the lanes hold plus those parked
+// in the warp's queue in shared memory).  If shading would not fill the
+// waiting lanes, their collisions are parked and they take primary rays.  The
+// lane-owned loop above serves whatever each lane happens to need, about 9 of
+// 32 lanes in its shading code; here nearly all waiting lanes run it.
+//
+// Pixels whose rays cannot meet the volume's box (FrameDD::cull, formed on the
+// host) issue no paths; they add their miss colour where they are found (three
+// quarters of the 1080p frame around a cube).
+//
+// Bound: instruction issue and fetch.  Against the lane-owned loop on the 512^3
+// 1080p 64-spp frame (ncu on 8 spp): warp instructions 1.65 -> 1.05 G, 11.1 -> 16.8
+// of 32 lanes a instruction, 14.5 -> 10.0 ms; 256^2 x 16 spp of a 64^3 volume, where
+// a pixel's waves no longer wait for one another, 1.0 -> 0.24 ms; 64 mixed jobs
+// 41 -> 29 ms.  Shading at once in every pass that waits on samples: the steps
+// that end inside a macrocell wait for one another too (4 -> 14 lanes a sample).
+constexpr float kPathOccluded = 0.f, kPathLit = 1.f, kPathMissed = 2.f;  // outcome in the ring entry's w
+
+// A warp's shared memory: everything its lanes do not need between two
+// service passes, so that the tracing loop keeps only the ray in registers.
+struct StreamWarp {
+  // parked collisions: (P, t), (direction before the zero fix-up, ring index),
+  // (TF colour, seed low), seed high
+  float4 qA[32], qB[32], qC[32];
+  unsigned qD[32];
+  float4 entry[kStreamSlotPaths];  // the slot being retired
+  uint2 seed[32];  // RNG seed of each lane's ray, after its set-up
+  // the unit's pixels, and which of them issue paths
+  int2 pixel[32];
+  unsigned char pathPixel[32];
+  // slots, by ring position: paths not done, job, first pixel in chunk order,
+  // pixels, first wave, waves, pixels that issue paths (bit = pixel - first), their
+  // number's reciprocal (slotWave)
+  int left[kStreamSlots], job[kStreamSlots], first[kStreamSlots], count[kStreamSlots];
+  int wave[kStreamSlots], waves[kStreamSlots];
+  unsigned mask[kStreamSlots], inv[kStreamSlots];
+  unsigned head, tail;  // slots [head, tail) are in use
+  int nextPath, pathsLeft;  // of the newest slot: the next path to issue, paths not issued
+  int unitJob, unitFirst, unitCount, unitWave, unitWavesLeft;  // the unit being issued; its waves in no slot yet
+  unsigned unitMask;
+  int exhausted;   // no unit is left
+  unsigned error;  // error bits
+  unsigned long long culledRays;  // rays of pixels that issue no paths
+};
+
+// Ring entries bypass L1: a warp writes each once and reads it once.
+DEV void ringStore(float4 *p, float4 v) {
+  asm volatile("st.global.cg.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+DEV void ringStoreW(float4 *p, float w) { asm volatile("st.global.cg.f32 [%0], %1;" ::"l"(&p->w), "f"(w) : "memory"); }
+DEV void ringFetch(float4 *shared, const float4 *p) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(p) : "memory");
+}
+DEV void ringFetchWait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The pixel's rays cannot meet the volume's bounds: its square lies beyond an
+// edge of their projection (cullEdges in bn_api.cpp, with its error margin).
+DEV bool pixelMisses(const FrameDD &fr, int ix, int iy) {
+  const float x = ix + .5f, y = iy + .5f;
+  bool out = false;
+#pragma unroll
+  for (int e = 0; e < kCullEdges; e++) out = out || fr.cull[e].x * x + fr.cull[e].y * y + fr.cull[e].z > 0.f;
+  return out;
+}
+
+// Path i of a slot with n = popc(mask) issuing pixels is wave i / n: i < 64 and
+// n <= 32, so i ceil(2^16 / n) / 2^16 (error below 64/2^16 < 1/32) is exact.
+DEV int slotWave(const StreamWarp &sw, int s, int i) { return (int)((unsigned)i * sw.inv[s] >> 16); }
+
+// Opens slot `tail`: the next waves of the current unit, or the first ones of
+// the frame's next unit.  Called by the whole warp, with work left.  Returns
+// the number of its pixels that issue paths; with 0 the slot holds all waves
+// of the unit, to be retired at once (tail is not advanced), or there was no
+// unit left (sw.exhausted).
+template <bool BATCH>
+DEV int openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs, int numChunks,
+                 int unitSplit, LaunchCounters *ctr, StreamWarp &sw) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int unitPixels = 32 >> unitSplit;
+  if (sw.unitWavesLeft == 0) {
+    unsigned u = 0, ab = 0;
+    if (lane == 0) {
+      u = atomicAdd(&ctr->nextPixel, 1u);
+      ab = *(volatile unsigned *)&ctr->abort;
+    }
+    u = __shfl_sync(FULL, u, 0);
+    ab = __shfl_sync(FULL, ab, 0);
+    if (ab || u >= (unsigned)numChunks << unitSplit) {
+      if (lane == 0) {
+        sw.exhausted = 1;
+        if (ab) sw.error |= ERR_ABORTED;
+      }
+      __syncwarp();
+      return 0;
+    }
+    const int sub = (int)(u & ((1u << unitSplit) - 1u));
+    int c = (int)(u >> unitSplit);  // the chunk
+    int j = 0;
+    if (BATCH) {  // last job whose first chunk is <= c
+      int lo = 0, hi = numJobs - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (chunkStart[mid] <= c) lo = mid; else hi = mid - 1;
+      }
+      j = lo;
+    }
+    const FrameDD &fr = jobs[j].fr;
+    if (!BATCH && fr.partCount > 1)  // this rank's k-th chunk -> the frame's chunk
+      c = (c / kPartTileChunks * fr.partCount + fr.partRank) * kPartTileChunks + c % kPartTileChunks;
+    const int first = (c - (BATCH ? chunkStart[j] : 0)) * kChunk + sub * unitPixels;
+    const int count = min(unitPixels, fr.width * fr.height - first);  // <= 0: the last chunk's missing pixels
+    int ix = 0, iy = 0;
+    bool issues = false;
+    if (lane < count) {
+      chunkPixel(fr, first + lane, ix, iy);
+      issues = !pixelMisses(fr, ix, iy);
+    }
+    const unsigned m = __ballot_sync(FULL, issues);
+    if (lane < count) sw.pixel[lane] = make_int2(ix, iy);
+    if (issues) sw.pathPixel[__popc(m & ((1u << lane) - 1u))] = (unsigned char)lane;
+    if (lane == 0) {
+      sw.culledRays += (unsigned long long)(max(count, 0) - __popc(m)) * (unsigned)fr.spp;
+      sw.unitJob = j;
+      sw.unitFirst = first;
+      sw.unitCount = count;
+      sw.unitMask = m;
+      sw.unitWave = 0;
+      sw.unitWavesLeft = fr.spp;
+    }
+    __syncwarp();
+  }
+  const int n = __popc(sw.unitMask);
+  __syncwarp();
+  if (lane == 0) {
+    const int s = (int)(sw.tail & (kStreamSlots - 1u));
+    const int waves = n ? min(kStreamSlotPaths / unitPixels, sw.unitWavesLeft) : sw.unitWavesLeft;
+    sw.left[s] = sw.pathsLeft = waves * n;
+    sw.job[s] = sw.unitJob;
+    sw.first[s] = sw.unitFirst;
+    sw.count[s] = sw.unitCount;
+    sw.mask[s] = sw.unitMask;
+    sw.inv[s] = (65535u + (unsigned)n) / (unsigned)max(n, 1);
+    sw.wave[s] = sw.unitWave;
+    sw.waves[s] = waves;
+    sw.nextPath = 0;
+    sw.unitWave += waves;
+    sw.unitWavesLeft -= waves;
+    if (n) sw.tail++;
+  }
+  __syncwarp();
+  return n;
+}
+
+// Adds the outcomes of a slot's paths to its pixels' accumulators (shadeRays.cu:996-1040),
+// one lane per pixel, in wave order.  Called by the whole warp.
+DEV void retireSlot(const FrameDD &fr, StreamWarp &sw, int s, const float4 *ring) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = sw.mask[s];
+  const int n = __popc(m);
+  int waves = sw.waves[s], accumID = fr.accumID0 + sw.wave[s];
+  // the slot's entries to shared memory: one round trip to L2, not one a wave
+  const int total = n * waves;
+  for (int i = lane; i < total && i < kStreamSlotPaths; i += 32) ringFetch(&sw.entry[i], ring + s * kStreamSlotPaths + i);
+  int ix = 0, iy = 0;
+  bool mine = lane < sw.count[s];
+  if (mine) chunkPixel(fr, sw.first[s] + lane, ix, iy);
+  const int64_t pix = (int64_t)iy * fr.width + ix;
+  mine = mine && BNB_IN(pix, (long long)fr.width * fr.height);
+  const bool cmp = fr.comp != nullptr;
+  float4 acc = mine && accumID > 0 ? fr.accum[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 comp = mine && cmp && accumID > 0 ? fr.comp[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 bg = missColor(fr, iy);
+  const bool issues = (m >> lane) & 1u;
+  // a pixel that issues no paths, with a miss that adds alpha 1 and no colour:
+  // whole numbers below 2^24 add without rounding, so its waves are one
+  // addition (which leaves the compensation terms as they are)
+  const bool whole = !issues && bg.w == 1.f && !(bg.x > 0.f) && !(bg.y > 0.f) && !(bg.z > 0.f) && accumID > 0 &&
+                     acc.w >= 0.f && acc.w == truncf(acc.w) && acc.w <= 8388608.f && waves <= 8388608;
+  if (whole) acc.w += (float)waves;
+  if (!mine || whole) waves = 0;
+  const float4 *entry = sw.entry + (issues ? __popc(m & ((1u << lane) - 1u)) : 0);
+  ringFetchWait();
+  __syncwarp();
+#pragma unroll 1
+  for (; waves > 0; waves--, accumID++) {
+    float4 f = *entry;
+    if (issues) entry += n;
+    const bool missed = !issues || f.w == kPathMissed;
+    float w = 1.f;
+    if (missed) {
+      const float clampMax = 10.f * (1 + accumID);
+      f.x = fmin_(bg.x, clampMax);
+      f.y = fmin_(bg.y, clampMax);
+      f.z = fmin_(bg.z, clampMax);
+      w = bg.w;
+    } else if (f.w == kPathOccluded) {
+      f.x = f.y = f.z = 0.f;
+    }
+    if (accumID == 0) {  // generation 0 sets: the miss colour, emission-absorption's colour, else black
+      acc = make_float4(0.f, 0.f, 0.f, w);
+      comp = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (missed || fr.emissionAbsorption) {
+        acc.x = f.x;
+        acc.y = f.y;
+        acc.z = f.z;
+        continue;
+      }
+    } else if (w > 0.f) {
+      accAdd(acc.w, comp.w, w, cmp);
+    }
+    if (f.x > 0.f) accAdd(acc.x, comp.x, f.x, cmp);
+    if (f.y > 0.f) accAdd(acc.y, comp.y, f.y, cmp);
+    if (f.z > 0.f) accAdd(acc.z, comp.z, f.z, cmp);
+  }
+  if (!mine) return;
+  fr.accum[pix] = acc;
+  if (cmp) fr.comp[pix] = comp;
+}
+
+// True only if the free flight of this draw, RN(-log(1 - draw) / maj), reaches
+// the end of the remaining range `left` whatever its rounding: with the
+// logarithm within 2e-6 of the exact kernels' (a quotient of 2 ulp in a series
+// of one sign), a margin of 1e-5 covers it and the roundings of maj * left.
+// A majorant <= 0 or NaN, a zero draw or an underflowing product give false or
+// a true that holds exactly, so such steps go through the exact evaluation.
+template <int LOG>
+DEV bool leavesCell(float draw, float maj, float left) {
+  float l;
+  if (LOG) {
+    l = -logPortable(1.f - draw);
+  } else {
+    const float u = 1.f - draw;
+    const float f = __fdividef(draw, u + 1.f);  // -(u - 1) / (u + 1)
+    const float f2 = f * f;
+    const float s = f + (1.f / 3.f) * (f * f2) + (1.f / 5.f) * (f * f2 * f2);
+    l = s + s;
+  }
+  return maj > 0.f && l * (1.f - 1e-5f) > maj * left;
+}
+
+template <int T, bool BATCH, int LOG>
+DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs, int numChunks,
+                    const SchedDD &sd, LaunchCounters *ctr, float4 *ring, StreamWarp &sw, const float4 *sTF,
+                    const float *u8lut) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  if (lane == 0) {
+    sw.head = sw.tail = 0;
+    sw.nextPath = sw.pathsLeft = sw.unitWavesLeft = sw.exhausted = 0;
+    sw.error = 0;
+    sw.culledRays = 0;
+  }
+  __syncwarp();
+
+  // lane state.  A collision's TF colour waits in ts.tNext, which a ray that
+  // has ended no longer needs; bit 64 of ts.bits marks a shadow ray.
+  unsigned nSamples = 0, nVisits = 0, nRays = 0;
+  int parked = 0;  // warp-uniform: collisions in the queue
+  int phase = LP_IDLE;
+  int job = 0;
+  int path = 0;  // ring index
+  TraceState ts{};
+  float draw = 0.f;  // the free-flight draw of a lane in LP_SAMPLE
+  unsigned steps = 0;
+
+  while (true) {
+    // between two service passes a lane traces at most one ray (< 2^24
+    // counter increments), so 32-bit lane counters flushed from 2^31 on never wrap
+    if ((nSamples | nVisits | nRays) >= 0x80000000u) {
+      atomicAdd(&ctr->samples, (unsigned long long)nSamples);
+      atomicAdd(&ctr->mcVisits, (unsigned long long)nVisits);
+      atomicAdd(&ctr->rays, (unsigned long long)nRays);
+      nSamples = nVisits = nRays = 0;
+    }
+    // ------------------------------------------------------------------
+    // 1. paths that are done write their outcome (a shadow ray's fragment is
+    //    in its entry since it was spawned); a primary ray's collision stays
+    //    LP_HIT, to be shaded
+    // ------------------------------------------------------------------
+    if (phase == LP_HIT || phase == LP_ENDED) {
+      const bool shadow = ts.bits & 64;
+      bool done = true;
+      if (phase == LP_HIT && !shadow) {
+        const FrameDD &fr = jobs[BATCH ? job : 0].fr;
+        done = fr.emissionAbsorption;
+        if (done) {
+          const int s = path / kStreamSlotPaths;
+          const float clampMax = 10.f * (1 + fr.accumID0 + sw.wave[s] + slotWave(sw, s, path % kStreamSlotPaths));
+          ringStore(ring + path, make_float4(fmin_(ts.tNext.x, clampMax), fmin_(ts.tNext.y, clampMax),
+                                             fmin_(ts.tNext.z, clampMax), kPathLit));
+        }
+      } else if (!shadow || phase == LP_HIT) {
+        ringStoreW(ring + path, shadow ? kPathOccluded : kPathMissed);
+      }
+      if (done) {
+        atomicSub(&sw.left[path / kStreamSlotPaths], 1);
+        phase = LP_IDLE;
+      }
+    }
+    __syncwarp();
+    // ------------------------------------------------------------------
+    // 2. what the waiting lanes do next: shade if their collisions and the
+    //    parked ones fill them all (or no path can be issued), else issue
+    //    primary rays, their collisions parked
+    // ------------------------------------------------------------------
+    unsigned waiting = __ballot_sync(FULL, phase == LP_IDLE || phase == LP_HIT);
+    const unsigned holding = __ballot_sync(FULL, phase == LP_HIT);
+    const bool shading = __popc(holding) + parked >= __popc(waiting) ||
+                         (sw.pathsLeft == 0 && ((sw.unitWavesLeft == 0 && sw.exhausted) ||
+                                                (sw.tail - sw.head == kStreamSlots && sw.left[sw.head & (kStreamSlots - 1u)] != 0)));
+    int pixelX = 0, pixelY = 0, wave = 0;
+    if (!shading) {
+      if (phase == LP_HIT) {
+        const int q = parked + __popc(holding & below);
+        const uint2 seed = sw.seed[lane];
+        sw.qA[q] = make_float4(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z, ts.t);
+        sw.qB[q] = make_float4((ts.bits & 8) ? 0.f : ts.dir.x, (ts.bits & 16) ? 0.f : ts.dir.y,
+                               (ts.bits & 32) ? 0.f : ts.dir.z, __int_as_float(path));
+        sw.qC[q] = make_float4(ts.tNext.x, ts.tNext.y, ts.tNext.z, __uint_as_float(seed.x));
+        sw.qD[q] = seed.y;
+        phase = LP_IDLE;
+      }
+      parked += __popc(holding);
+      __syncwarp();
+    }
+    // ------------------------------------------------------------------
+    // 3. slots whose paths are all done retire, oldest first; paths go to the
+    //    waiting lanes, opening slots as needed
+    // ------------------------------------------------------------------
+    while (true) {
+      int s = (int)(sw.head & (kStreamSlots - 1u));
+      const bool oldest = sw.head != sw.tail && sw.left[s] == 0;
+      if (!oldest) {
+        if (shading || !waiting) break;
+        if (sw.pathsLeft > 0) {
+          s = (int)((sw.tail - 1u) & (kStreamSlots - 1u));
+          const int rank = __popc(waiting & below);
+          const int take = min(__popc(waiting), sw.pathsLeft);
+          const bool mine = ((waiting >> lane) & 1u) && rank < take;
+          if (mine) {
+            const int i = sw.nextPath + rank;
+            const int k = slotWave(sw, s, i);
+            const int2 p = sw.pixel[sw.pathPixel[i - k * __popc(sw.mask[s])]];
+            pixelX = p.x;
+            pixelY = p.y;
+            wave = sw.wave[s] + k;
+            path = s * kStreamSlotPaths + i;
+            if (BATCH) job = sw.job[s];
+            phase = LP_NEWSAMPLE;
+          }
+          waiting &= ~__ballot_sync(FULL, mine);
+          if (lane == 0) {
+            sw.nextPath += take;
+            sw.pathsLeft -= take;
+          }
+          __syncwarp();
+          continue;
+        }
+        if ((sw.unitWavesLeft == 0 && sw.exhausted) || sw.tail - sw.head == kStreamSlots) break;
+        s = (int)(sw.tail & (kStreamSlots - 1u));
+        if (openSlot<BATCH>(jobs, chunkStart, numJobs, numChunks, sd.unitSplit, ctr, sw) != 0 || sw.exhausted) continue;
+      }
+      retireSlot(jobs[BATCH ? sw.job[s] : 0].fr, sw, s, ring);
+      __syncwarp();
+      if (oldest && lane == 0) sw.head++;
+      __syncwarp();
+    }
+    if (shading) {
+      // 4. shading: the lanes' own collisions, and parked ones for the others
+      const unsigned empty = waiting & ~holding;
+      const int rank = __popc(empty & below);
+      bool shade = phase == LP_HIT;
+      float3 P = f3(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z);
+      // the ray's direction before traceBegin's zero fix-up
+      float3 dir = f3((ts.bits & 8) ? 0.f : ts.dir.x, (ts.bits & 16) ? 0.f : ts.dir.y, (ts.bits & 32) ? 0.f : ts.dir.z);
+      float tHit = ts.t;
+      float3 rgb = ts.tNext;
+      uint2 seed = sw.seed[lane];
+      if (((empty >> lane) & 1u) && rank < parked) {
+        const int q = parked - 1 - rank;
+        const float4 a = sw.qA[q], b = sw.qB[q], c = sw.qC[q];
+        P = f3(a.x, a.y, a.z);
+        tHit = a.w;
+        dir = f3(b.x, b.y, b.z);
+        path = __float_as_int(b.w);
+        rgb = f3(c.x, c.y, c.z);
+        seed = make_uint2(__float_as_uint(c.w), sw.qD[q]);
+        if (BATCH) job = sw.job[path / kStreamSlotPaths];
+        shade = true;
+      }
+      parked -= min(parked, __popc(empty));
+      __syncwarp();
+      if (shade) {
+        const JobDD &J = jobs[BATCH ? job : 0];
+        const int s = path / kStreamSlotPaths;
+        const float clampMax = 10.f * (1 + J.fr.accumID0 + sw.wave[s] + slotWave(sw, s, path % kStreamSlotPaths));
+        uint64_t raySeed = (uint64_t)seed.x | ((uint64_t)seed.y << 32);
+        float3 frag;
+        ts.bits = 64;
+        phase = LP_HIT;  // no shadow ray goes out: as an occluded one
+        if (shadeVolumeHit(J.v, J.fr, P, tHit, dir, rgb, clampMax, raySeed, ts.org, ts.dir, ts.rayTMax, frag)) {
+          ringStore(ring + path, make_float4(frag.x, frag.y, frag.z, kPathLit));
+          sw.seed[lane] = make_uint2((unsigned)raySeed, (unsigned)(raySeed >> 32));
+          phase = LP_BEGIN;
+        }
+      }
+    } else if (phase == LP_NEWSAMPLE) {
+      const FrameDD &fr = jobs[BATCH ? job : 0].fr;
+      uint64_t raySeed;
+      primaryRay(fr, pixelX, pixelY, fr.accumID0 + wave, ts.org, ts.dir, ts.rayTMax, raySeed);
+      sw.seed[lane] = make_uint2((unsigned)raySeed, (unsigned)(raySeed >> 32));
+      ts.bits = 0;
+      phase = LP_BEGIN;
+    }
+    const bool moreWork = parked > 0 || sw.pathsLeft > 0 ||
+                          ((sw.unitWavesLeft > 0 || !sw.exhausted) && sw.tail - sw.head < kStreamSlots);
+    // no lane at work, nothing parked or to issue: every path is done, and so
+    // every slot retired
+    if (!__ballot_sync(FULL, phase != LP_IDLE) && !moreWork) break;
+    const JobDD &J = jobs[BATCH ? job : 0];
+    const VolumeDD &v = J.v;
+    // ------------------------------------------------------------------
+    // 5. ray set-up
+    // ------------------------------------------------------------------
+    if (phase == LP_BEGIN) {
+      const uint2 seed = sw.seed[lane];
+      uint64_t raySeed = (uint64_t)seed.x | ((uint64_t)seed.y << 32);
+      const int shadow = ts.bits;
+      nRays++;
+      steps = 0;
+      phase = traceBegin(v, ts, ts.org, ts.dir, ts.rayTMax, raySeed) ? LP_CELL : LP_ENDED;
+      ts.bits = phase == LP_CELL ? ts.bits | shadow : shadow;
+      sw.seed[lane] = make_uint2((unsigned)raySeed, (unsigned)(raySeed >> 32));
+    }
+    while (true) {
+      // ------------------------------------------------------------------
+      // 6. next macrocell with a non-zero majorant (DDA.h:172-200,
+      //    MCAccelerator.h:596-612)
+      // ------------------------------------------------------------------
+      if (phase == LP_CELL) {
+        while (true) {
+          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
+          // cell indices are inside the grid here and the grid has < 2^31 cells
+          const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
+          const bool occupied = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z) &&
+                                ((__ldg(v.mcOccupied + (ci >> 5)) >> (ci & 31)) & 1u);
+          nVisits++;
+          if (!occupied) {  // majorant == 0
+            if (!ddaStep(v, ts, tClosest)) { phase = LP_ENDED; break; }
+            if (++steps > (1u << 22)) { atomicOr(&sw.error, ERR_ITER_CAP); phase = LP_ENDED; break; }
+          } else {
+            ts.maj = __ldg(v.majorants + ci);
+            ts.t = ts.rayT0 + ts.nextCellBegin;
+            ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
+            phase = LP_WOODCOCK;
+            break;
+          }
+        }
+      }
+      // ------------------------------------------------------------------
+      // 7. the free-flight draw of a Woodcock step (Volume.h:180-201).  Most
+      //    draws leave the macrocell; the distance itself then does not
+      //    matter, so an approximate logarithm decides with a margin, and
+      //    only the draws that may end inside wait for 8, where the exact
+      //    distance is formed.
+      // ------------------------------------------------------------------
+      if (phase == LP_WOODCOCK) {
+        draw = rngFloat(ts.rng);
+        steps++;
+        if (leavesCell<LOG>(draw, ts.maj, ts.tUpper - ts.t)) {
+          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
+          phase = ddaStep(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+          if (steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
+            atomicOr(&sw.error, ERR_ITER_CAP);
+            phase = LP_ENDED;
+          }
+        } else {
+          phase = LP_SAMPLE;
+        }
+      }
+      const int nWalking = __popc(__ballot_sync(FULL, phase == LP_CELL));
+      if (nWalking > 32 - sd.sampleBatch) continue;
+      // ------------------------------------------------------------------
+      // 8. the steps that end inside their macrocell: sample and accept or
+      //    reject.  Every lane that got here since the last time takes part
+      //    (right after each draw it would be 4 of 32 on average).
+      // ------------------------------------------------------------------
+      if (phase == LP_SAMPLE) {
+        ts.t += LOG ? (-logPortable(1.f - draw) / ts.maj) : (-fastLog(1.f - draw) / ts.maj);
+        if (ts.t >= ts.tUpper) {
+          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
+          phase = ddaStep(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+        } else {
+          phase = LP_WOODCOCK;
+          const float3 P = f3(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z);
+          const float s = sampleJob<T>(v, P, u8lut);
+          nSamples++;
+          float w = 0.f, f = 0.f;
+          int idx = 0;
+          if (!isnan(s)) {
+            tfLocate(v, s, idx, f);
+            if (!BNB_IN(idx, v.tfN - 1)) idx = 0;
+            const float w0 = BATCH ? __ldg(&v.tf[idx].w) : sTF[idx].w;
+            const float w1 = BATCH ? __ldg(&v.tf[idx + 1].w) : sTF[idx + 1].w;
+            w = __fmul_rn(lerp_l(f, w0, w1), v.baseDensity);
+          }
+          if (w >= rngFloat(ts.rng) * ts.maj) {
+            // the TF colour (a shadow ray's is never read)
+            ts.tNext = f3(0.f, 0.f, 0.f);
+            if (!isnan(s)) {
+              const float4 a = BATCH ? __ldg(&v.tf[idx]) : sTF[idx];
+              const float4 b = BATCH ? __ldg(&v.tf[idx + 1]) : sTF[idx + 1];
+              ts.tNext = f3(lerp_l(f, a.x, b.x), lerp_l(f, a.y, b.y), lerp_l(f, a.z, b.z));
+            }
+            phase = LP_HIT;
+          }
+        }
+        if (steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
+          atomicOr(&sw.error, ERR_ITER_CAP);
+          phase = LP_ENDED;
+        }
+      }
+      const bool moving = phase == LP_WOODCOCK || phase == LP_CELL;
+      const int nMoving = __popc(__ballot_sync(FULL, moving));
+      const int nWaiting = __popc(__ballot_sync(FULL, !moving && (phase != LP_IDLE || moreWork)));
+      if (nMoving == 0 || nWaiting >= sd.serviceBatch) break;
+    }
+  }
+
+  // counters: warp reduction in 64 bits, one atomic per warp
+  unsigned long long wSamples = nSamples, wVisits = nVisits, wRays = nRays;
+  for (int o = 16; o > 0; o >>= 1) {
+    wSamples += __shfl_down_sync(FULL, wSamples, o);
+    wVisits += __shfl_down_sync(FULL, wVisits, o);
+    wRays += __shfl_down_sync(FULL, wRays, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&ctr->samples, wSamples);
+    atomicAdd(&ctr->mcVisits, wVisits);
+    atomicAdd(&ctr->rays, wRays + sw.culledRays);
+    if (sw.error) atomicOr(&ctr->errorFlags, (unsigned long long)sw.error);
+  }
+}
+
+// The warp's slice of the launch's ring memory.
+DEV float4 *streamRing(float4 *ring) {
+  return ring + (size_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kStreamRing;
+}
+// The unorm8 table, for the kernels that read it.
+template <int T>
+DEV void fillU8Table(float *u8lut) {
+  if (T == VOX_U8 || T < 0)
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) u8lut[i] = __fdiv_rn((float)i * 1.f, 255.f);
+}
+
+template <int T, int LOG>
+__global__ void __launch_bounds__(kRenderMaxThreads, kRenderMinBlocks)
+    streamKernel(const __grid_constant__ JobDD job, const __grid_constant__ SchedDD sd, LaunchCounters *ctr,
+                 float4 *ring) {
+  extern __shared__ float4 sTF[];
+  __shared__ float u8lut[T == VOX_U8 ? 256 : 1];
+  __shared__ StreamWarp sWarp[kRenderMaxThreads / 32];
+  for (int i = threadIdx.x; i < job.v.tfN; i += blockDim.x) sTF[i] = job.v.tf[i];
+  fillU8Table<T>(u8lut);
+  __syncthreads();
+  int numChunks = (job.fr.width * job.fr.height + kChunk - 1) / kChunk;
+  if (job.fr.partCount > 1) numChunks = partitionChunks(numChunks, job.fr.partRank, job.fr.partCount);
+  streamLoop<T, false, LOG>(&job, nullptr, 1, numChunks, sd, ctr, streamRing(ring), sWarp[threadIdx.x >> 5], sTF, u8lut);
+}
+
+// A table of jobs in global memory.  T: the voxel type every job has, or -1
+// (mixed: a switch per sample).  Free-flight distances with fastLog only;
+// batches with an exact-log job run the extended kernel, which chooses per job.
+template <int T>
+__global__ void __launch_bounds__(kRenderMaxThreads, kRenderMinBlocks)
+    streamBatchKernel(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs,
+                      const __grid_constant__ SchedDD sd, LaunchCounters *ctr, float4 *ring) {
+  __shared__ float u8lut[T == VOX_U8 || T < 0 ? 256 : 1];
+  __shared__ StreamWarp sWarp[kRenderMaxThreads / 32];
+  fillU8Table<T>(u8lut);
+  __syncthreads();
+  streamLoop<T, true, 0>(jobs, chunkStart, numJobs, __ldg(chunkStart + numJobs), sd, ctr, streamRing(ring),
+                         sWarp[threadIdx.x >> 5], nullptr, u8lut);
 }
 
 // ---------------------------------------------------------------------------
@@ -2315,34 +2998,8 @@ __global__ void __launch_bounds__(kAQThreads, kAQMinBlocks)
       if (lane == 0 && doneNow) atomicSub(&sh.live, __popc(doneNow));
       // A4: primary rays (generateRays.cu:71-243)
       if (phase == LP_NEWSAMPLE) {
-        const int accumID = fr.accumID0 + kk;
-        const unsigned uAcc = (unsigned)accumID;
-        uint64_t rnd = rngSeed2((unsigned)px + (unsigned)W * uAcc, (unsigned)py + (unsigned)H * uAcc);
-        raySeed = rngSeed2((unsigned)px + uAcc * (unsigned)W, (uint32_t)py);
-        const float pixel_u = (accumID == 0) ? .5f : rngFloat(rnd);
-        const float pixel_v = (accumID == 0) ? .5f : rngFloat(rnd);
-        const float image_u = ((px + pixel_u) / float(W));
-        const float image_v = ((py + pixel_v) / float(H));
-        const float aspect = fr.aspect;  // W / float(H), formed on the host
-        const float su = 1.f * aspect * (image_u - .5f), sv = 1.f * (image_v - .5f);
-        float3 d = f3(fr.dir00.x + su * fr.dirdu.x + sv * fr.dirdv.x, fr.dir00.y + su * fr.dirdu.y + sv * fr.dirdv.y,
-                      fr.dir00.z + su * fr.dirdu.z + sv * fr.dirdv.z);
-        d = normalize3(d);
-        float3 o = fr.lens00;
-        tMax = 1e30f;
-        if (fr.cutPlane.w > -1e28f) {
-          const float3 N = f3(fr.cutPlane.x, fr.cutPlane.y, fr.cutPlane.z);
-          const float dist_org = dot3(N, o) + fr.cutPlane.w;
-          const float denom = dot3(N, d);
-          if (dist_org >= 0.f) {
-            if (denom < 0.f) tMax = fmin_(tMax, -dist_org / denom);
-          } else {
-            if (denom > 0.f) {
-              const float te = -dist_org / denom;
-              o = f3(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
-            } else tMax = 0.f;
-          }
-        }
+        float3 o, d;
+        primaryRay(fr, px, py, fr.accumID0 + kk, o, d, tMax, raySeed);
         meta &= ~16;  // a primary ray
         nRays++;
         org = o;
@@ -2420,23 +3077,20 @@ __global__ void __launch_bounds__(kAQThreads, kAQMinBlocks)
   }
 }
 
+#ifndef BNB_FAST_MATH
 // T: the voxel type every job of the batch has, or -1 (mixed: a switch per sample)
 template <int T, int EXT, int CMP>
-__global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2     ? kRenderMinBlocksIso
-                                                     : EXT        ? kRenderMinBlocksExt
-                                                     : CMP == 1   ? kRenderMinBlocksMixedComp
-                                                                  : kRenderMinBlocks)
+__global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2 ? kRenderMinBlocksIso : kRenderMinBlocksExt)
     renderBatchKernel(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs, const __grid_constant__ SchedDD sd,
                       LaunchCounters *ctr) {
   __shared__ float u8lut[256];
   __shared__ float sIsoBuf[EXT >= 2 ? kRenderMaxThreads / 32 * kIsoBufPerWarp : 1];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) u8lut[i] = __fdiv_rn((float)i * 1.f, 255.f);
   __syncthreads();
-  // plain batch kernels draw free-flight distances with fastLog only; batches
-  // with an exact-log job run the extended kernel, which chooses per job
-  renderLoop<T, true, EXT ? 2 : 0, EXT, CMP>(jobs, chunkStart, numJobs, __ldg(chunkStart + numJobs), sd, ctr, nullptr,
-                                             u8lut, EXT >= 2 ? sIsoBuf + (threadIdx.x >> 5) * kIsoBufPerWarp : nullptr);
+  renderLoop<T, true, 2, EXT, CMP>(jobs, chunkStart, numJobs, __ldg(chunkStart + numJobs), sd, ctr, nullptr, u8lut,
+                                   EXT >= 2 ? sIsoBuf + (threadIdx.x >> 5) * kIsoBufPerWarp : nullptr);
 }
+#endif  // !BNB_FAST_MATH
 
 // Field samples and transfer-function lookups at given points
 // (bnxVolumeSample): the structured sampler (NaN outside) and sampleAndMap
@@ -2602,19 +3256,63 @@ cudaError_t launchMapMajorants(const VolumeDD &v, const float2 *ranges, float *m
 }
 #endif  // !BNB_FAST_MATH
 
+// log2 of the units a 32-pixel chunk is cut into.  A slot holds 64 paths of one
+// unit: fewer pixels with more waves, or more with fewer.  Larger units retire
+// with fewer idle lanes; smaller ones spread a small frame over more warps.
+// Measured (kernel ms at 32 / 16 / 8 pixels a unit): 512^3 1080p 64 spp 10.15 /
+// 10.04 / 10.33; 1024^2 4 spp 0.641 / 0.639 / 0.727; 1279x719 1 spp 0.152 / 0.212 /
+// 0.348 (slots of 32, 16 and 8 paths); 256^2 16 spp, 2048 chunks over 4144 warps,
+// 0.585 / 0.370 / 0.242.
+static int unitSplitFor(long long chunks, int spp, int warps) {
+  if (spp < 4) return 0;
+  return spp >= 8 && chunks < 4LL * warps ? 2 : 1;
+}
+
+// Blocks of a launch: bps per SM (0: as many as fit), at most the warps that
+// have a ring.
+template <typename K>
+static cudaError_t streamGrid(K kern, int bps, int tpb, size_t smem, const StreamRing &ring, int &blocks) {
+  if (!ring.ptr) return cudaErrorInvalidValue;
+  if (bps <= 0) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, smem) != cudaSuccess) return cudaGetLastError();
+    bps = occ > 0 ? occ : 1;
+  }
+  blocks = (int)std::min<int64_t>((int64_t)smCount() * bps, ring.warps / (tpb / 32));
+  return blocks > 0 ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <int T>
-static cudaError_t launchRenderT(const VolumeDD &v, const FrameDD &fr, const SchedDD &sd, LaunchCounters *ctr,
-                                 int bps, int tpb, cudaStream_t s) {
+static cudaError_t launchStreamT(const VolumeDD &v, const FrameDD &fr, SchedDD sd, LaunchCounters *ctr, int bps,
+                                 int tpb, cudaStream_t s, const StreamRing &ring) {
+  const size_t smem = (size_t)v.tfN * sizeof(float4);
+  auto kern = fr.exactLog ? streamKernel<T, 1> : streamKernel<T, 0>;
+  if (smem > 32 * 1024 &&  // with the kernel's static shared memory above the 48 KB a launch may use unasked
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return cudaGetLastError();
+  int blocks = 0;
+  const cudaError_t e = streamGrid(kern, bps, tpb, smem, ring, blocks);
+  if (e != cudaSuccess) return e;
+  sd.unitSplit = unitSplitFor(((long long)fr.width * fr.height + kChunk - 1) / kChunk, fr.spp, blocks * (tpb / 32));
+  JobDD job;
+  job.v = v;
+  job.fr = fr;
+  kern<<<blocks, tpb, smem, s>>>(job, sd, ctr, ring.ptr);
+  return cudaGetLastError();
+}
+
+#ifndef BNB_FAST_MATH
+// The lane-owned kernels: extended jobs, and plain ones on the path that has
+// no ring memory (the no-allocation entry point, without compensated sums).
+template <int T>
+static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, const SchedDD &sd, LaunchCounters *ctr,
+                                int bps, int tpb, cudaStream_t s) {
   const size_t smem = (size_t)v.tfN * sizeof(float4);
   const bool pvms = fr.maxVolumeBounces > 0 || v.pv.enabled;
   const int ext = v.iso.enabled ? (pvms ? 2 : 3) : pvms ? 1 : 0;
   // kernels with and without compensated sums
   const bool cmp = fr.comp != nullptr;
-#ifdef BNB_FAST_MATH
-  if (ext) return cudaErrorInvalidValue;  // the fast-math object holds the plain kernels only
-  auto kern = cmp ? (fr.exactLog ? renderKernel<T, 1, 0, 2> : renderKernel<T, 0, 0, 2>)
-                  : (fr.exactLog ? renderKernel<T, 1, 0, 0> : renderKernel<T, 0, 0, 0>);
-#else
+  if (ext == 0 && cmp) return cudaErrorInvalidValue;
   // isosurfaces without volume bounces or principled volumes: the smaller
   // EXT 3 kernel unless the job keeps compensated sums
   auto kern = ext == 3 && !cmp ? (fr.exactLog ? renderKernel<T, 1, 3, 0> : renderKernel<T, 0, 3, 0>)
@@ -2622,9 +3320,7 @@ static cudaError_t launchRenderT(const VolumeDD &v, const FrameDD &fr, const Sch
                                 : (fr.exactLog ? renderKernel<T, 1, 2, 0> : renderKernel<T, 0, 2, 0>))
               : ext == 1 ? (cmp ? (fr.exactLog ? renderKernel<T, 1, 1, 2> : renderKernel<T, 0, 1, 2>)
                                 : (fr.exactLog ? renderKernel<T, 1, 1, 0> : renderKernel<T, 0, 1, 0>))
-              : cmp ? (fr.exactLog ? renderKernel<T, 1, 0, 2> : renderKernel<T, 0, 0, 2>)
-                    : (fr.exactLog ? renderKernel<T, 1, 0, 0> : renderKernel<T, 0, 0, 0>);
-#endif
+                         : (fr.exactLog ? renderKernel<T, 1, 0, 0> : renderKernel<T, 0, 0, 0>);
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return cudaGetLastError();
@@ -2638,6 +3334,19 @@ static cudaError_t launchRenderT(const VolumeDD &v, const FrameDD &fr, const Sch
   job.fr = fr;
   kern<<<smCount() * bps, tpb, smem, s>>>(job, sd, ctr);
   return cudaGetLastError();
+}
+#endif  // !BNB_FAST_MATH
+
+template <int T>
+static cudaError_t launchRenderT(const VolumeDD &v, const FrameDD &fr, const SchedDD &sd, LaunchCounters *ctr,
+                                 int bps, int tpb, cudaStream_t s, const StreamRing &ring) {
+  const bool ext = v.iso.enabled || fr.maxVolumeBounces > 0 || v.pv.enabled;
+#ifdef BNB_FAST_MATH
+  if (ext) return cudaErrorInvalidValue;  // the fast-math object holds the plain kernels only
+#else
+  if (ext || !ring.ptr) return launchLanesT<T>(v, fr, sd, ctr, bps, tpb, s);
+#endif
+  return launchStreamT<T>(v, fr, sd, ctr, bps, tpb, s, ring);
 }
 
 template <int T>
@@ -2668,17 +3377,18 @@ cudaError_t launchRenderRegrouped(const VolumeDD &v, const FrameDD &fr, LaunchCo
 }
 
 cudaError_t launchRender(const VolumeDD &v, const FrameDD &fr, LaunchCounters *ctr, int bps, int tpb, cudaStream_t s,
-                         const SchedDD &sd) {
+                         const SchedDD &sd, const StreamRing &ring) {
   if (tpb <= 0) tpb = 128;
   switch (v.type) {
-  case VOX_F32: return launchRenderT<VOX_F32>(v, fr, sd, ctr, bps, tpb, s);
-  case VOX_U8: return launchRenderT<VOX_U8>(v, fr, sd, ctr, bps, tpb, s);
-  case VOX_F16: return launchRenderT<VOX_F16>(v, fr, sd, ctr, bps, tpb, s);
-  case VOX_U16: return launchRenderT<VOX_U16>(v, fr, sd, ctr, bps, tpb, s);
-  default: return launchRenderT<VOX_BF16>(v, fr, sd, ctr, bps, tpb, s);
+  case VOX_F32: return launchRenderT<VOX_F32>(v, fr, sd, ctr, bps, tpb, s, ring);
+  case VOX_U8: return launchRenderT<VOX_U8>(v, fr, sd, ctr, bps, tpb, s, ring);
+  case VOX_F16: return launchRenderT<VOX_F16>(v, fr, sd, ctr, bps, tpb, s, ring);
+  case VOX_U16: return launchRenderT<VOX_U16>(v, fr, sd, ctr, bps, tpb, s, ring);
+  default: return launchRenderT<VOX_BF16>(v, fr, sd, ctr, bps, tpb, s, ring);
   }
 }
 
+#ifndef BNB_FAST_MATH
 template <int EXT, int CMP>
 static auto batchKernelFor(int voxelType) {
   switch (voxelType) {
@@ -2690,6 +3400,7 @@ static auto batchKernelFor(int voxelType) {
   default: return renderBatchKernel<-1, EXT, CMP>;
   }
 }
+#endif  // !BNB_FAST_MATH
 
 // A batch of at most kParamJobs plain jobs passed as a kernel parameter
 // (constant bank) instead of a table in global memory: the jobs' fields are
@@ -2700,41 +3411,33 @@ struct JobTableParam {
   JobDD jobs[kParamJobs];
   int chunkStart[kParamJobs + 1];
 };
-template <int T, int CMP>
-__global__ void __launch_bounds__(kRenderMaxThreads, CMP == 1 ? kRenderMinBlocksMixedComp : kRenderMinBlocks)
-    renderBatchParamKernel(const __grid_constant__ JobTableParam tab, int numJobs, const __grid_constant__ SchedDD sd,
-                           LaunchCounters *ctr) {
-  __shared__ float u8lut[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) u8lut[i] = __fdiv_rn((float)i * 1.f, 255.f);
+static_assert(sizeof(JobTableParam) + sizeof(SchedDD) + 32 <= 32764, "a kernel's parameters are at most 32764 bytes");
+template <int T>
+__global__ void __launch_bounds__(kRenderMaxThreads, kRenderMinBlocks)
+    streamBatchParamKernel(const __grid_constant__ JobTableParam tab, int numJobs, const __grid_constant__ SchedDD sd,
+                           LaunchCounters *ctr, float4 *ring) {
+  __shared__ float u8lut[T == VOX_U8 || T < 0 ? 256 : 1];
+  __shared__ StreamWarp sWarp[kRenderMaxThreads / 32];
+  fillU8Table<T>(u8lut);
   __syncthreads();
-  renderLoop<T, true, 0, 0, CMP>(tab.jobs, tab.chunkStart, numJobs, tab.chunkStart[numJobs], sd, ctr, nullptr, u8lut,
-                                 nullptr);
-}
-template <int CMP>
-static auto batchParamKernelFor(int voxelType) {
-  switch (voxelType) {
-  case VOX_F32: return renderBatchParamKernel<VOX_F32, CMP>;
-  case VOX_U8: return renderBatchParamKernel<VOX_U8, CMP>;
-  case VOX_F16: return renderBatchParamKernel<VOX_F16, CMP>;
-  case VOX_U16: return renderBatchParamKernel<VOX_U16, CMP>;
-  case VOX_BF16: return renderBatchParamKernel<VOX_BF16, CMP>;
-  default: return renderBatchParamKernel<-1, CMP>;
-  }
+  streamLoop<T, true, 0>(tab.jobs, tab.chunkStart, numJobs, tab.chunkStart[numJobs], sd, ctr, streamRing(ring),
+                         sWarp[threadIdx.x >> 5], nullptr, u8lut);
 }
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
-                                    LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, const SchedDD &sd,
-                                    int voxelType, int compensated) {
+                                    LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd, int voxelType,
+                                    const StreamRing &ring) {
   if (numJobs < 1 || numJobs > kParamJobs) return cudaErrorInvalidValue;
   if (tpb <= 0) tpb = 128;
-  auto kern = compensated == 2   ? batchParamKernelFor<2>(voxelType)
-              : compensated == 1 ? batchParamKernelFor<1>(voxelType)
-                                 : batchParamKernelFor<0>(voxelType);
-  if (bps <= 0) {
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, 0) != cudaSuccess)
-      return cudaGetLastError();
-    bps = occ > 0 ? occ : 1;
-  }
+  auto kern = voxelType == VOX_F32    ? streamBatchParamKernel<VOX_F32>
+              : voxelType == VOX_U8   ? streamBatchParamKernel<VOX_U8>
+              : voxelType == VOX_F16  ? streamBatchParamKernel<VOX_F16>
+              : voxelType == VOX_U16  ? streamBatchParamKernel<VOX_U16>
+              : voxelType == VOX_BF16 ? streamBatchParamKernel<VOX_BF16>
+                                      : streamBatchParamKernel<-1>;
+  int blocks = 0;
+  const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
+  if (e != cudaSuccess) return e;
+  sd.unitSplit = unitSplitFor(hostChunkStart[numJobs], 8, blocks * (tpb / 32));
   // host staging of the 31 KB parameter (the launch copies it); one launch
   // at a time fills it
   static JobTableParam tab;
@@ -2742,27 +3445,34 @@ cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkS
   std::lock_guard<std::mutex> l(m);
   memcpy(tab.jobs, hostJobs, numJobs * sizeof(JobDD));
   memcpy(tab.chunkStart, hostChunkStart, (numJobs + 1) * sizeof(int));
-  kern<<<smCount() * bps, tpb, 0, s>>>(tab, numJobs, sd, ctr);
+  kern<<<blocks, tpb, 0, s>>>(tab, numJobs, sd, ctr, ring.ptr);
   return cudaGetLastError();
 }
 
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, LaunchCounters *ctr, int bps,
-                              int tpb, cudaStream_t s, const SchedDD &sd, int extended, int voxelType,
-                              int compensated) {
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
+                              LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd, int extended, int voxelType, int compensated,
+                              const StreamRing &ring) {
   if (tpb <= 0) tpb = 128;
+  if (!extended) {
+    auto kern = voxelType == VOX_F32    ? streamBatchKernel<VOX_F32>
+                : voxelType == VOX_U8   ? streamBatchKernel<VOX_U8>
+                : voxelType == VOX_F16  ? streamBatchKernel<VOX_F16>
+                : voxelType == VOX_U16  ? streamBatchKernel<VOX_U16>
+                : voxelType == VOX_BF16 ? streamBatchKernel<VOX_BF16>
+                                        : streamBatchKernel<-1>;
+    int blocks = 0;
+  const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
+    if (e != cudaSuccess) return e;
+    sd.unitSplit = unitSplitFor(numChunks, 8, blocks * (tpb / 32));
+    kern<<<blocks, tpb, 0, s>>>(jobs, chunkStart, numJobs, sd, ctr, ring.ptr);
+    return cudaGetLastError();
+  }
 #ifdef BNB_FAST_MATH
-  if (extended) return cudaErrorInvalidValue;  // the fast-math object holds the plain kernels only
-  auto kern = compensated == 2   ? batchKernelFor<0, 2>(voxelType)
-              : compensated == 1 ? batchKernelFor<0, 1>(voxelType)
-                                 : batchKernelFor<0, 0>(voxelType);
+  return cudaErrorInvalidValue;  // the fast-math object holds the plain kernels only
 #else
   auto kern = extended == 3 && !compensated ? batchKernelFor<3, 0>(voxelType)
-              : extended >= 2    ? (compensated ? batchKernelFor<2, 1>(voxelType) : batchKernelFor<2, 0>(voxelType))
-              : extended         ? (compensated ? batchKernelFor<1, 1>(voxelType) : batchKernelFor<1, 0>(voxelType))
-              : compensated == 2 ? batchKernelFor<0, 2>(voxelType)
-              : compensated == 1 ? batchKernelFor<0, 1>(voxelType)
-                                 : batchKernelFor<0, 0>(voxelType);
-#endif
+              : extended >= 2 ? (compensated ? batchKernelFor<2, 1>(voxelType) : batchKernelFor<2, 0>(voxelType))
+                              : (compensated ? batchKernelFor<1, 1>(voxelType) : batchKernelFor<1, 0>(voxelType));
   if (bps <= 0) {
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, tpb, 0) != cudaSuccess)
@@ -2771,6 +3481,7 @@ cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJ
   }
   kern<<<smCount() * bps, tpb, 0, s>>>(jobs, chunkStart, numJobs, sd, ctr);
   return cudaGetLastError();
+#endif
 }
 
 cudaError_t launchSampleProbe(const VolumeDD &v, const float3 *P, int n, float *scalar, float4 *rgba, cudaStream_t s) {
@@ -2935,7 +3646,7 @@ cudaError_t launchRenderNoAlloc(VolumeDD v, FrameDD fr, int fmt, void *color, in
   if (e != cudaSuccess) return e;
   e = launchOccupancy(majorants, n, occupied, s);
   if (e != cudaSuccess) return e;
-  e = launchRender(v, fr, ctr, 0, 0, s);
+  e = launchRender(v, fr, ctr, 0, 0, s, SchedDD(), StreamRing());
   if (e != cudaSuccess) return e;
   return launchResolve(fr.accum, fr.width * fr.height, fr.accumID0 + fr.spp, fmt, color, s);
 }

@@ -428,6 +428,7 @@ struct Context {
   cudaStream_t ownStream = nullptr;
   cudaStream_t stream = nullptr;
   LaunchCounters *dCounters = nullptr;
+  StreamRing ring;  // of this context's plain render launches (kept: 16 KB per resident warp)
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   int blocksPerSM = 0, threadsPerBlock = 128;
   SchedDD sched;
@@ -455,6 +456,10 @@ struct Context {
     stream = ownStream;
     ck(deviceMalloc((void **)&dCounters, sizeof(LaunchCounters)), "cudaMalloc counters");
     ck(cudaMemset(dCounters, 0, sizeof(LaunchCounters)), "cudaMemset");
+    int sms = 0;
+    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    ring.warps = sms * kStreamWarpsPerSM;
+    ck(deviceMalloc((void **)&ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4)), "cudaMalloc path rings");
     for (auto &e : ev) ck(cudaEventCreate(&e), "cudaEventCreate");
   }
   ~Context() {
@@ -468,6 +473,7 @@ struct Context {
     handles.clear();
     for (auto &e : ev) if (e) cudaEventDestroy(e);
     if (dCounters) cudaFree(dCounters);
+    if (ring.ptr) cudaFree(ring.ptr);
     if (ownStream) cudaStreamDestroy(ownStream);
     cudaGetLastError();  // nothing of a destroyed context may leak into later calls
   }
