@@ -80,8 +80,8 @@ struct VolumeDD {
 
 struct DirLightDD {
   float3 toLight;       // -normalize(direction)  (DirLight.cu:11-20, shadeRays.cu:180)
-  float radiance;
-  float3 color;
+  float weight;         // the largest component of rad
+  float3 rad;           // color * radiance
 };
 
 // One frame's worth of render parameters (Camera::DD, Renderer::DD,

@@ -475,6 +475,22 @@ DEV bool ddaStep(const VolumeDD &v, TraceState &ts, float tClosest) {
   return true;
 }
 
+// ddaStep without branches: an axis that does not step keeps its values, and
+// stepping the others after the grid is left has no effect on a ray that ended.
+DEV bool leaveCell(const VolumeDD &v, TraceState &ts, float tClosest) {
+  ts.nextCellBegin = tClosest;
+  const bool ax = ts.tNext.x == tClosest, ay = ts.tNext.y == tClosest, az = ts.tNext.z == tClosest;
+  if (ax) ts.tNext.x += ts.tStep.x;
+  if (ay) ts.tNext.y += ts.tStep.y;
+  if (az) ts.tNext.z += ts.tStep.z;
+  if (ax) ts.cx += (ts.bits & 1) * 2 - 1;
+  if (ay) ts.cy += (ts.bits & 2) - 1;
+  if (az) ts.cz += (ts.bits & 4) / 2 - 1;
+  // an index only leaves the grid by the step just taken: to -1 or its size
+  return (unsigned)ts.cx < (unsigned)v.mcDims.x && (unsigned)ts.cy < (unsigned)v.mcDims.y &&
+         (unsigned)ts.cz < (unsigned)v.mcDims.z;
+}
+
 struct LightSample {
   float3 dir, radiance;
   float pdf;
@@ -565,58 +581,49 @@ DEV bool sampleLights(const FrameDD &fr, uint64_t &random, LightSample &ls, bool
   float dlsWeight = 0.f;
   float3 dDir = f3(0.f, 0.f, 0.f), dRad = f3(0.f, 0.f, 0.f);
   if (fr.numDirLights > 0) {
-    int lID[2];
-    float w[2];
-    float sumW = 0.f;
-    for (int i = 0; i < 2; i++) {
-      lID[i] = min(int(rngFloat(random) * fr.numDirLights), fr.numDirLights - 1);
-      w[i] = 0.f;
-      const DirLightDD &L = fr.dirLights[lID[i]];
-      float3 rad = f3(L.color.x * L.radiance, L.color.y * L.radiance, L.color.z * L.radiance);
-      float weight = nZero ? 1.f : dot3(L.toLight, N);
-      if (!nZero && weight <= 1e-3f) continue;
-      weight *= fmax_(fmax_(rad.x, rad.y), rad.z);
-      if (weight <= 1e-3f) continue;
-      w[i] = weight;
-      sumW += weight;
+    // a reservoir of two lights drawn uniformly, weighted by their radiance
+    // (and, on a surface, the cosine)
+    const int l0 = min(int(rngFloat(random) * fr.numDirLights), fr.numDirLights - 1);
+    const int l1 = min(int(rngFloat(random) * fr.numDirLights), fr.numDirLights - 1);
+    float w0 = fr.dirLights[l0].weight, w1 = fr.dirLights[l1].weight;
+    if (!nZero) {
+      const float c0 = dot3(fr.dirLights[l0].toLight, N), c1 = dot3(fr.dirLights[l1].toLight, N);
+      w0 = c0 <= 1e-3f ? 0.f : c0 * w0;
+      w1 = c1 <= 1e-3f ? 0.f : c1 * w1;
     }
+    if (w0 <= 1e-3f) w0 = 0.f;
+    if (w1 <= 1e-3f) w1 = 0.f;
+    const float sumW = w0 + w1;
     if (sumW != 0.f) {
       float r = rngFloat(random) * sumW;
-      int i = 0;
-      while (i < 2 && r >= w[i]) { r -= w[i]; ++i; }
-      if (i < 2) {
-        const DirLightDD &L = fr.dirLights[lID[i]];
+      const bool second = r >= w0;
+      if (second) r -= w0;
+      if (!(second && r >= w1)) {
+        const DirLightDD &L = fr.dirLights[second ? l1 : l0];
+        const float w = second ? w1 : w0;
         dDir = L.toLight;
-        const float den = w[i] / sumW * fr.dirLightPick;  // (2.f / float(numDirLights)), formed on the host
-        dRad = f3(L.color.x * L.radiance * 1.f / den, L.color.y * L.radiance * 1.f / den,
-                  L.color.z * L.radiance * 1.f / den);
-        if (w[i] != 0.f) dlsWeight = fmax_(fmax_(dRad.x, dRad.y), dRad.z);
+        const float den = w / sumW * fr.dirLightPick;  // (2.f / float(numDirLights)), formed on the host
+        dRad = f3(L.rad.x / den, L.rad.y / den, L.rad.z / den);
+        if (w != 0.f) dlsWeight = fmax_(fmax_(dRad.x, dRad.y), dRad.z);
       }
     }
   }
   float sumWeights = 0.f + dlsWeight + elsWeight + 0.f;
   if (sumWeights == 0.f) return false;
-  elsWeight *= 1.f / sumWeights;
-  const float alsWeight = 0.f * (1.f / sumWeights);
-  dlsWeight *= 1.f / sumWeights;
-  const float plsWeight = 0.f * (1.f / sumWeights);
+  const float rcpSum = 1.f / sumWeights;
+  elsWeight *= rcpSum;
+  const float alsWeight = 0.f * rcpSum;
+  dlsWeight *= rcpSum;
+  const float plsWeight = 0.f * rcpSum;
   const float r = rngFloat(random);
   if (r <= alsWeight) return false;  // area-light slot of an empty light list: pdf 0
-  if (r <= alsWeight + elsWeight) {
-    const float s = 1.f / elsWeight;
-    ls.dir = eDir;
-    ls.radiance = f3(eRad * s, eRad * s, eRad * s);
-    ls.pdf = nZero ? kOneOverFourPi : 1.f / (2.f * ONE_PI_F);
-    needsMIS = true;
-    return true;
-  }
-  if (r <= alsWeight + elsWeight + plsWeight) return false;
-  if (dlsWeight == 0.f) return false;
-  const float s = 1.f / dlsWeight;
-  ls.dir = dDir;
-  ls.radiance = f3(dRad.x * s, dRad.y * s, dRad.z * s);
-  ls.pdf = kInf;
-  isDir = true;
+  needsMIS = r <= alsWeight + elsWeight;  // the environment
+  if (!needsMIS && (r <= alsWeight + elsWeight + plsWeight || dlsWeight == 0.f)) return false;
+  isDir = !needsMIS;
+  const float s = 1.f / (isDir ? dlsWeight : elsWeight);
+  ls.dir = isDir ? dDir : eDir;
+  ls.radiance = f3((isDir ? dRad.x : eRad) * s, (isDir ? dRad.y : eRad) * s, (isDir ? dRad.z : eRad) * s);
+  ls.pdf = isDir ? kInf : nZero ? kOneOverFourPi : 1.f / (2.f * ONE_PI_F);
   return true;
 }
 
@@ -1175,7 +1182,7 @@ DEV bool shadeVolumeHit(const VolumeDD &v, const FrameDD &fr, float3 P, float tH
   float3 fv = f3(fpdf * alb.x, fpdf * alb.y, fpdf * alb.z);
   if (!(fpdf > 0.f) || fmax_(fmax_(fv.x, fv.y), fv.z) < 1e-4f) return false;
   fv = f3(fmin_(fv.x, 13.f), fmin_(fv.y, 13.f), fmin_(fv.z, 13.f));
-  const float ip = isinf(ls.pdf) ? 1.f : (1.f / ls.pdf);
+  const float ip = isDir ? 1.f : 1.f / kOneOverFourPi;  // 1 / ls.pdf
   const float3 tp = f3(1.f * ip * fv.x * ls.radiance.x * 1.f, 1.f * ip * fv.y * ls.radiance.y * 1.f,
                        1.f * ip * fv.z * ls.radiance.z * 1.f);
   float misWeight = 1.f;
@@ -1877,11 +1884,8 @@ struct StreamWarp {
   int left[kStreamSlots], job[kStreamSlots], first[kStreamSlots], count[kStreamSlots];
   int wave[kStreamSlots], waves[kStreamSlots];
   unsigned mask[kStreamSlots], inv[kStreamSlots];
-  unsigned head, tail;  // slots [head, tail) are in use
-  int nextPath, pathsLeft;  // of the newest slot: the next path to issue, paths not issued
   int unitJob, unitFirst, unitCount, unitWave, unitWavesLeft;  // the unit being issued; its waves in no slot yet
   unsigned unitMask;
-  int exhausted;   // no unit is left
   unsigned error;  // error bits
   unsigned long long culledRays;  // rays of pixels that issue no paths
 };
@@ -1910,14 +1914,35 @@ DEV bool pixelMisses(const FrameDD &fr, int ix, int iy) {
 // n <= 32, so i ceil(2^16 / n) / 2^16 (error below 64/2^16 < 1/32) is exact.
 DEV int slotWave(const StreamWarp &sw, int s, int i) { return (int)((unsigned)i * sw.inv[s] >> 16); }
 
-// Opens slot `tail`: the next waves of the current unit, or the first ones of
-// the frame's next unit.  Called by the whole warp, with work left.  Returns
-// the number of its pixels that issue paths; with 0 the slot holds all waves
-// of the unit, to be retired at once (tail is not advanced), or there was no
-// unit left (sw.exhausted).
+// The warp's control word, the same in every lane: the oldest slot, slots in
+// use, paths of the newest slot not issued and the next one of them, whether
+// slots are left to open, and the parked collisions.
+struct StreamCtl {
+  unsigned bits = 1u << 23;
+  DEV int head() const { return bits & (kStreamSlots - 1u); }
+  DEV int used() const { return (bits >> 4) & 31u; }
+  DEV int pathsLeft() const { return (bits >> 9) & 127u; }
+  DEV int nextPath() const { return (bits >> 16) & 127u; }
+  DEV bool more() const { return (bits >> 23) & 1u; }
+  DEV int parked() const { return bits >> 24; }
+  DEV int newest() const { return (bits + (bits >> 4) - 1u) & (kStreamSlots - 1u); }
+  DEV int next() const { return (bits + (bits >> 4)) & (kStreamSlots - 1u); }
+  DEV bool canIssue() const { return pathsLeft() > 0 || (more() && used() < (int)kStreamSlots); }
+  DEV void park(int n) { bits += (unsigned)n << 24; }
+  DEV void retireHead() { bits = (bits & ~15u) - 16u + ((bits + 1u) & (kStreamSlots - 1u)); }
+  DEV void issue(int n) { bits += ((unsigned)n << 16) - ((unsigned)n << 9); }
+  DEV void open(int paths) { bits = ((bits & ~((127u << 9) | (127u << 16))) | (unsigned)paths << 9) + 16u; }
+  DEV void setMore(bool m) { bits = (bits & ~(1u << 23)) | (m ? 1u << 23 : 0u); }
+};
+static_assert(kStreamSlots <= 16 && (kStreamSlots & (kStreamSlots - 1)) == 0 && kStreamSlotPaths <= 127, "StreamCtl's fields");
+
+// Opens slot ctl.next(): the next waves of the current unit, or the first ones
+// of the frame's next unit.  Called by the whole warp, with ctl.more().  Returns
+// false if the slot has no path: it then holds all waves of the unit, to be
+// retired at once (it is not in use), or no unit was left (!ctl.more()).
 template <bool BATCH>
-DEV int openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs, int numChunks,
-                 int unitSplit, LaunchCounters *ctr, StreamWarp &sw) {
+DEV bool openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkStart, int numJobs, int numChunks,
+                 int unitSplit, LaunchCounters *ctr, StreamWarp &sw, StreamCtl &ctl) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int unitPixels = 32 >> unitSplit;
@@ -1930,12 +1955,9 @@ DEV int openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkSt
     u = __shfl_sync(FULL, u, 0);
     ab = __shfl_sync(FULL, ab, 0);
     if (ab || u >= (unsigned)numChunks << unitSplit) {
-      if (lane == 0) {
-        sw.exhausted = 1;
-        if (ab) sw.error |= ERR_ABORTED;
-      }
-      __syncwarp();
-      return 0;
+      if (ab && lane == 0) sw.error |= ERR_ABORTED;
+      ctl.setMore(false);
+      return false;
     }
     const int sub = (int)(u & ((1u << unitSplit) - 1u));
     int c = (int)(u >> unitSplit);  // the chunk
@@ -1973,12 +1995,11 @@ DEV int openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkSt
     }
     __syncwarp();
   }
-  const int n = __popc(sw.unitMask);
+  const int n = __popc(sw.unitMask), left = sw.unitWavesLeft, s = ctl.next();
+  const int waves = n ? min(kStreamSlotPaths / unitPixels, left) : left;
   __syncwarp();
   if (lane == 0) {
-    const int s = (int)(sw.tail & (kStreamSlots - 1u));
-    const int waves = n ? min(kStreamSlotPaths / unitPixels, sw.unitWavesLeft) : sw.unitWavesLeft;
-    sw.left[s] = sw.pathsLeft = waves * n;
+    sw.left[s] = waves * n;
     sw.job[s] = sw.unitJob;
     sw.first[s] = sw.unitFirst;
     sw.count[s] = sw.unitCount;
@@ -1986,13 +2007,12 @@ DEV int openSlot(const JobDD *__restrict__ jobs, const int *__restrict__ chunkSt
     sw.inv[s] = (65535u + (unsigned)n) / (unsigned)max(n, 1);
     sw.wave[s] = sw.unitWave;
     sw.waves[s] = waves;
-    sw.nextPath = 0;
     sw.unitWave += waves;
-    sw.unitWavesLeft -= waves;
-    if (n) sw.tail++;
+    sw.unitWavesLeft = left - waves;
   }
   __syncwarp();
-  return n;
+  if (n) ctl.open(waves * n);
+  return n != 0;
 }
 
 // Adds the outcomes of a slot's paths to its pixels' accumulators (shadeRays.cu:996-1040),
@@ -2074,7 +2094,9 @@ DEV bool leavesCell(float draw, float maj, float left) {
     l = -logPortable(1.f - draw);
   } else {
     const float u = 1.f - draw;
-    const float f = __fdividef(draw, u + 1.f);  // -(u - 1) / (u + 1)
+    float rcp;  // of a value in [1, 2]: within 1 ulp
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(u + 1.f));
+    const float f = draw * rcp;  // -(u - 1) / (u + 1)
     const float f2 = f * f;
     const float s = f + (1.f / 3.f) * (f * f2) + (1.f / 5.f) * (f * f2 * f2);
     l = s + s;
@@ -2090,8 +2112,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   if (lane == 0) {
-    sw.head = sw.tail = 0;
-    sw.nextPath = sw.pathsLeft = sw.unitWavesLeft = sw.exhausted = 0;
+    sw.unitWavesLeft = 0;
     sw.error = 0;
     sw.culledRays = 0;
   }
@@ -2100,7 +2121,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
   // lane state.  A collision's TF colour waits in ts.tNext, which a ray that
   // has ended no longer needs; bit 64 of ts.bits marks a shadow ray.
   unsigned nSamples = 0, nVisits = 0, nRays = 0;
-  int parked = 0;  // warp-uniform: collisions in the queue
+  StreamCtl ctl;
   int phase = LP_IDLE;
   int job = 0;
   int path = 0;  // ring index
@@ -2150,13 +2171,12 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
     // ------------------------------------------------------------------
     unsigned waiting = __ballot_sync(FULL, phase == LP_IDLE || phase == LP_HIT);
     const unsigned holding = __ballot_sync(FULL, phase == LP_HIT);
-    const bool shading = __popc(holding) + parked >= __popc(waiting) ||
-                         (sw.pathsLeft == 0 && ((sw.unitWavesLeft == 0 && sw.exhausted) ||
-                                                (sw.tail - sw.head == kStreamSlots && sw.left[sw.head & (kStreamSlots - 1u)] != 0)));
+    bool oldestDone = ctl.used() > 0 && sw.left[ctl.head()] == 0;
+    const bool shading = __popc(holding) + ctl.parked() >= __popc(waiting) || !(ctl.canIssue() || (ctl.more() && oldestDone));
     int pixelX = 0, pixelY = 0, wave = 0;
     if (!shading) {
       if (phase == LP_HIT) {
-        const int q = parked + __popc(holding & below);
+        const int q = ctl.parked() + __popc(holding & below);
         const uint2 seed = sw.seed[lane];
         sw.qA[q] = make_float4(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z, ts.t);
         sw.qB[q] = make_float4((ts.bits & 8) ? 0.f : ts.dir.x, (ts.bits & 16) ? 0.f : ts.dir.y,
@@ -2165,7 +2185,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
         sw.qD[q] = seed.y;
         phase = LP_IDLE;
       }
-      parked += __popc(holding);
+      ctl.park(__popc(holding));
       __syncwarp();
     }
     // ------------------------------------------------------------------
@@ -2173,17 +2193,16 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
     //    waiting lanes, opening slots as needed
     // ------------------------------------------------------------------
     while (true) {
-      int s = (int)(sw.head & (kStreamSlots - 1u));
-      const bool oldest = sw.head != sw.tail && sw.left[s] == 0;
-      if (!oldest) {
+      int s = ctl.head();
+      if (!oldestDone) {
         if (shading || !waiting) break;
-        if (sw.pathsLeft > 0) {
-          s = (int)((sw.tail - 1u) & (kStreamSlots - 1u));
+        if (ctl.pathsLeft() > 0) {
+          s = ctl.newest();
           const int rank = __popc(waiting & below);
-          const int take = min(__popc(waiting), sw.pathsLeft);
+          const int take = min(__popc(waiting), ctl.pathsLeft());
           const bool mine = ((waiting >> lane) & 1u) && rank < take;
           if (mine) {
-            const int i = sw.nextPath + rank;
+            const int i = ctl.nextPath() + rank;
             const int k = slotWave(sw, s, i);
             const int2 p = sw.pixel[sw.pathPixel[i - k * __popc(sw.mask[s])]];
             pixelX = p.x;
@@ -2194,21 +2213,19 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
             phase = LP_NEWSAMPLE;
           }
           waiting &= ~__ballot_sync(FULL, mine);
-          if (lane == 0) {
-            sw.nextPath += take;
-            sw.pathsLeft -= take;
-          }
-          __syncwarp();
+          ctl.issue(take);
           continue;
         }
-        if ((sw.unitWavesLeft == 0 && sw.exhausted) || sw.tail - sw.head == kStreamSlots) break;
-        s = (int)(sw.tail & (kStreamSlots - 1u));
-        if (openSlot<BATCH>(jobs, chunkStart, numJobs, numChunks, sd.unitSplit, ctr, sw) != 0 || sw.exhausted) continue;
+        if (!ctl.canIssue()) break;
+        s = ctl.next();
+        if (openSlot<BATCH>(jobs, chunkStart, numJobs, numChunks, sd.unitSplit, ctr, sw, ctl)) continue;
+        if (!ctl.more()) break;
+      } else {
+        ctl.retireHead();
       }
       retireSlot(jobs[BATCH ? sw.job[s] : 0].fr, sw, s, ring);
       __syncwarp();
-      if (oldest && lane == 0) sw.head++;
-      __syncwarp();
+      oldestDone = ctl.used() > 0 && sw.left[ctl.head()] == 0;
     }
     if (shading) {
       // 4. shading: the lanes' own collisions, and parked ones for the others
@@ -2221,6 +2238,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       float tHit = ts.t;
       float3 rgb = ts.tNext;
       uint2 seed = sw.seed[lane];
+      const int parked = ctl.parked();
       if (((empty >> lane) & 1u) && rank < parked) {
         const int q = parked - 1 - rank;
         const float4 a = sw.qA[q], b = sw.qB[q], c = sw.qC[q];
@@ -2233,7 +2251,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
         if (BATCH) job = sw.job[path / kStreamSlotPaths];
         shade = true;
       }
-      parked -= min(parked, __popc(empty));
+      ctl.park(-min(parked, __popc(empty)));
       __syncwarp();
       if (shade) {
         const JobDD &J = jobs[BATCH ? job : 0];
@@ -2257,8 +2275,7 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       ts.bits = 0;
       phase = LP_BEGIN;
     }
-    const bool moreWork = parked > 0 || sw.pathsLeft > 0 ||
-                          ((sw.unitWavesLeft > 0 || !sw.exhausted) && sw.tail - sw.head < kStreamSlots);
+    const bool moreWork = ctl.parked() > 0 || ctl.canIssue();
     // no lane at work, nothing parked or to issue: every path is done, and so
     // every slot retired
     if (!__ballot_sync(FULL, phase != LP_IDLE) && !moreWork) break;
@@ -2279,62 +2296,55 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
     }
     while (true) {
       // ------------------------------------------------------------------
-      // 6. next macrocell with a non-zero majorant (DDA.h:172-200,
-      //    MCAccelerator.h:596-612)
-      // ------------------------------------------------------------------
-      if (phase == LP_CELL) {
-        while (true) {
-          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-          // cell indices are inside the grid here and the grid has < 2^31 cells
-          const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
-          const bool occupied = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z) &&
-                                ((__ldg(v.mcOccupied + (ci >> 5)) >> (ci & 31)) & 1u);
-          nVisits++;
-          if (!occupied) {  // majorant == 0
-            if (!ddaStep(v, ts, tClosest)) { phase = LP_ENDED; break; }
-            if (++steps > (1u << 22)) { atomicOr(&sw.error, ERR_ITER_CAP); phase = LP_ENDED; break; }
-          } else {
-            ts.maj = __ldg(v.majorants + ci);
-            ts.t = ts.rayT0 + ts.nextCellBegin;
-            ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
-            phase = LP_WOODCOCK;
-            break;
-          }
-        }
-      }
-      // ------------------------------------------------------------------
-      // 7. the free-flight draw of a Woodcock step (Volume.h:180-201).  Most
-      //    draws leave the macrocell; the distance itself then does not
-      //    matter, so an approximate logarithm decides with a margin, and
-      //    only the draws that may end inside wait for 8, where the exact
+      // 6. one macrocell of every walking ray (DDA.h:172-200,
+      //    MCAccelerator.h:596-612): an empty one is left; in one with a
+      //    majorant the free-flight draw of a Woodcock step (Volume.h:180-201)
+      //    is taken.  Most draws leave the macrocell; the distance itself then
+      //    does not matter, so an approximate logarithm decides with a margin,
+      //    and only the draws that may end inside wait for 7, where the exact
       //    distance is formed.
       // ------------------------------------------------------------------
-      if (phase == LP_WOODCOCK) {
-        draw = rngFloat(ts.rng);
+      if (phase == LP_CELL || phase == LP_WOODCOCK) {
+        const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
+        bool leaves = false;
+        if (phase == LP_CELL) {
+          // cell indices are inside the grid here and the grid has < 2^31 cells
+          const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
+          const bool in = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z);
+          const float maj = in ? __ldg(v.majorants + ci) : 0.f;
+          leaves = maj == 0.f;
+          nVisits++;
+          if (!leaves) {
+            ts.maj = maj;
+            ts.t = ts.rayT0 + ts.nextCellBegin;
+            ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
+          }
+        }
         steps++;
-        if (leavesCell<LOG>(draw, ts.maj, ts.tUpper - ts.t)) {
-          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-          phase = ddaStep(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+        if (!leaves) {
+          draw = rngFloat(ts.rng);
+          leaves = leavesCell<LOG>(draw, ts.maj, ts.tUpper - ts.t);
+        }
+        phase = LP_SAMPLE;
+        if (leaves) {
+          phase = leaveCell(v, ts, tClosest) ? LP_CELL : LP_ENDED;
           if (steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
             atomicOr(&sw.error, ERR_ITER_CAP);
             phase = LP_ENDED;
           }
-        } else {
-          phase = LP_SAMPLE;
         }
       }
       const int nWalking = __popc(__ballot_sync(FULL, phase == LP_CELL));
       if (nWalking > 32 - sd.sampleBatch) continue;
       // ------------------------------------------------------------------
-      // 8. the steps that end inside their macrocell: sample and accept or
+      // 7. the steps that end inside their macrocell: sample and accept or
       //    reject.  Every lane that got here since the last time takes part
       //    (right after each draw it would be 4 of 32 on average).
       // ------------------------------------------------------------------
       if (phase == LP_SAMPLE) {
         ts.t += LOG ? (-logPortable(1.f - draw) / ts.maj) : (-fastLog(1.f - draw) / ts.maj);
-        if (ts.t >= ts.tUpper) {
-          const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-          phase = ddaStep(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+        if (ts.t >= ts.tUpper) {  // (the margin's few)
+          phase = leaveCell(v, ts, fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z)) ? LP_CELL : LP_ENDED;
         } else {
           phase = LP_WOODCOCK;
           const float3 P = f3(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z);
@@ -3259,13 +3269,13 @@ cudaError_t launchMapMajorants(const VolumeDD &v, const float2 *ranges, float *m
 // log2 of the units a 32-pixel chunk is cut into.  A slot holds 64 paths of one
 // unit: fewer pixels with more waves, or more with fewer.  Larger units retire
 // with fewer idle lanes; smaller ones spread a small frame over more warps.
-// Measured (kernel ms at 32 / 16 / 8 pixels a unit): 512^3 1080p 64 spp 10.15 /
-// 10.04 / 10.33; 1024^2 4 spp 0.641 / 0.639 / 0.727; 1279x719 1 spp 0.152 / 0.212 /
-// 0.348 (slots of 32, 16 and 8 paths); 256^2 16 spp, 2048 chunks over 4144 warps,
-// 0.585 / 0.370 / 0.242.
+// Measured (kernel ms at 32 / 16 / 8 pixels a unit): 512^3 1080p 64 spp 7.86 /
+// 7.78 / 8.08; 1024^2 4 spp 0.496 / 0.515 / 0.610; 1279x719 1 spp 0.134 / 0.196 /
+// 0.331 (slots of 32, 16 and 8 paths); 256^2 16 spp, 2048 chunks over 4144 warps,
+// 0.499 / 0.351 / 0.217.
 static int unitSplitFor(long long chunks, int spp, int warps) {
-  if (spp < 4) return 0;
-  return spp >= 8 && chunks < 4LL * warps ? 2 : 1;
+  if (spp < 8) return 0;
+  return chunks < 4LL * warps ? 2 : 1;
 }
 
 // Blocks of a launch: bps per SM (0: as many as fit), at most the warps that

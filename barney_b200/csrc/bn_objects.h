@@ -326,8 +326,8 @@ struct DirLight : Object {
     DirLightDD d;
     v3 dir = normalize(direction);
     d.toLight = make_float3(-dir.x, -dir.y, -dir.z);
-    d.color = F3(color);
-    d.radiance = std::isnan(irradiance) ? radiance : irradiance;
+    d.rad = F3(color * (std::isnan(irradiance) ? radiance : irradiance));
+    d.weight = fmaxf(fmaxf(d.rad.x, d.rad.y), d.rad.z);
     return d;
   }
 };
