@@ -125,8 +125,8 @@ struct JobDD {
 // busy lanes) need service -- shading, accumulation, a new ray -- and then
 // serves them together.
 struct SchedDD {
-  int serviceBatch = 22;
-  int sampleBatch = 26;  // streamed loop: lanes no longer walking before the steps among them are sampled
+  int serviceBatch = 0;    // 0: the launched kernel's own default
+  int sampleBatch = 26;    // lanes no longer walking before the steps among them are sampled
   int unitSplit = 0;  // streamed loop: log2 of the units a 32-pixel chunk is cut into (set by the launchers)
   int regrouped = 0;  // plain single-frame jobs: the regrouped kernel (launchRenderRegrouped) instead of renderLoop's
 };

@@ -491,6 +491,89 @@ DEV bool leaveCell(const VolumeDD &v, TraceState &ts, float tClosest) {
          (unsigned)ts.cz < (unsigned)v.mcDims.z;
 }
 
+// Lane phases of the render loop.
+enum LanePhase : int {
+  LP_IDLE = 0,      // no pixel
+  LP_NEWSAMPLE = 1, // the next wave of its pixel needs a primary ray
+  LP_CELL = 2,      // a ray needs its next macrocell with a non-zero majorant
+  LP_WOODCOCK = 3,  // inside a Woodcock range
+  LP_HIT = 4,       // collision found, waiting to be shaded
+  LP_ENDED = 5,     // ray left the grid (primary: background; shadow: reached the light)
+  LP_SAMPLE = 7,    // streamed loop: a Woodcock step that may end inside its range, waiting for its sample
+  LP_BEGIN = 6      // a new primary or shadow ray (ts.org, ts.dir, ts.rayTMax) needs its set-up
+};
+
+// True only if the free flight of this draw, RN(-log(1 - draw) / maj), reaches
+// the end of the remaining range `left` whatever its rounding: with the
+// logarithm within 2e-6 of the exact kernels' (a quotient of 2 ulp in a series
+// of one sign), a margin of 1e-5 covers it and the roundings of maj * left.
+// A majorant <= 0 or NaN, a zero draw or an underflowing product give false or
+// a true that holds exactly, so such steps go through the exact evaluation.
+DEV bool leavesCell(bool exactLog, float draw, float maj, float left) {
+  float l;
+  if (exactLog) {
+    l = -logPortable(1.f - draw);
+  } else {
+    const float u = 1.f - draw;
+    float rcp;  // of a value in [1, 2]: within 1 ulp
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(u + 1.f));
+    const float f = draw * rcp;  // -(u - 1) / (u + 1)
+    const float f2 = f * f;
+    const float s = f + (1.f / 3.f) * (f * f2) + (1.f / 5.f) * (f * f2 * f2);
+    l = s + s;
+  }
+  return maj > 0.f && l * (1.f - 1e-5f) > maj * left;
+}
+
+// One macrocell of a walking ray (LP_CELL: at a cell's start; LP_WOODCOCK: inside
+// its range; DDA.h:172-200, MCAccelerator.h:596-612): an empty one is left; in
+// one with a majorant the free-flight draw of a Woodcock step (Volume.h:180-201)
+// is taken.  Most draws leave the macrocell; the distance itself then does not
+// matter, so an approximate logarithm decides with a margin, and only the draws
+// that may end inside become LP_SAMPLE, where the exact distance is formed.
+// ISO: a ray with a surface hit (bit 64 of ts.bits) ends at the first occupied
+// macrocell that starts at or beyond it.  Returns true at the iteration cap.
+template <bool ISO>
+DEV bool walkCell(const VolumeDD &v, bool exactLog, TraceState &ts, int &phase, float &draw, unsigned &steps,
+                  unsigned &nVisits) {
+  const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
+  bool leaves = false;
+  if (phase == LP_CELL) {
+    // cell indices are inside the grid here and the grid has < 2^31 cells.  The
+    // majorant itself is loaded, not the occupancy bit: its L2 latency against
+    // one more load, and a dependent one, in every occupied cell (512^3 frame
+    // 8.0 -> 7.75 ms, one with 90 % empty cells 3.50 -> 3.62 ms)
+    const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
+    const bool in = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z);
+    const float maj = in ? __ldg(v.majorants + ci) : 0.f;
+    leaves = maj == 0.f;
+    nVisits++;
+    if (!leaves) {
+      if (ISO && (ts.bits & 64) && ts.rayT0 + ts.nextCellBegin >= ts.rayTMax) {
+        phase = LP_ENDED;
+        return false;
+      }
+      ts.maj = maj;
+      ts.t = ts.rayT0 + ts.nextCellBegin;
+      ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
+    }
+  }
+  steps++;
+  if (!leaves) {
+    draw = rngFloat(ts.rng);
+    leaves = leavesCell(exactLog, draw, ts.maj, ts.tUpper - ts.t);
+  }
+  phase = LP_SAMPLE;
+  if (leaves) {
+    phase = leaveCell(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+    if (steps > (1u << 22)) {  // end this ray as if it left the grid
+      phase = LP_ENDED;
+      return true;
+    }
+  }
+  return false;
+}
+
 struct LightSample {
   float3 dir, radiance;
   float pdf;
@@ -899,17 +982,6 @@ DEV float lambertPdf(float3 Ng, float3 wi) {
   return fmax_(dot3(wi, N), 0.f) * kOneOverPi;
 }
 
-// Lane phases of the render loop.
-enum LanePhase : int {
-  LP_IDLE = 0,      // no pixel
-  LP_NEWSAMPLE = 1, // the next wave of its pixel needs a primary ray
-  LP_CELL = 2,      // a ray needs its next macrocell with a non-zero majorant
-  LP_WOODCOCK = 3,  // inside a Woodcock range
-  LP_HIT = 4,       // collision found, waiting to be shaded
-  LP_ENDED = 5,     // ray left the grid (primary: background; shadow: reached the light)
-  LP_SAMPLE = 7,    // streamed loop: a Woodcock step that may end inside its range, waiting for its sample
-  LP_BEGIN = 6      // a new primary or shadow ray (ts.org, ts.dir, ts.rayTMax) needs its set-up
-};
 
 constexpr int kChunk = 32;  // pixels a warp takes at a time (one 8x4 tile)
 
@@ -1202,6 +1274,45 @@ DEV bool shadeVolumeHit(const VolumeDD &v, const FrameDD &fr, float3 P, float tH
   return true;
 }
 
+// The pixel's rays cannot meet the volume's bounds: its square lies beyond an
+// edge of their projection (cullEdges in bn_api.cpp, with its error margin).
+DEV bool pixelMisses(const FrameDD &fr, int ix, int iy) {
+  const float x = ix + .5f, y = iy + .5f;
+  bool out = false;
+#pragma unroll
+  for (int e = 0; e < kCullEdges; e++) out = out || fr.cull[e].x * x + fr.cull[e].y * y + fr.cull[e].z > 0.f;
+  return out;
+}
+
+// All waves of a pixel whose rays cannot meet the volume: the miss colour of
+// every wave (shadeRays.cu:996-1040).  Not inlined, so that the render loop
+// keeps its registers.
+__device__ __noinline__ void missPixel(const FrameDD &fr, int ix, int iy) {
+  const int64_t pix = (int64_t)iy * fr.width + ix;
+  if (!BNB_IN(pix, (long long)fr.width * fr.height)) return;
+  const bool cmp = fr.comp != nullptr;
+  const float4 bg = missColor(fr, iy);
+  float4 acc = fr.accumID0 > 0 ? fr.accum[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 comp = cmp && fr.accumID0 > 0 ? fr.comp[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int k = 0; k < fr.spp; k++) {
+    const int accumID = fr.accumID0 + k;
+    const float clampMax = 10.f * (1 + accumID);
+    const float fx = fmin_(bg.x, clampMax), fy = fmin_(bg.y, clampMax), fz = fmin_(bg.z, clampMax);
+    if (accumID == 0) {
+      acc = make_float4(fx, fy, fz, bg.w);
+      comp = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      if (bg.w > 0.f) accAdd(acc.w, comp.w, bg.w, cmp);
+      if (fx > 0.f) accAdd(acc.x, comp.x, fx, cmp);
+      if (fy > 0.f) accAdd(acc.y, comp.y, fy, cmp);
+      if (fz > 0.f) accAdd(acc.z, comp.z, fz, cmp);
+    }
+  }
+  fr.accum[pix] = acc;
+  if (cmp) fr.comp[pix] = comp;
+}
+
 // The render loop shared by the single-frame kernel (one job, read from a
 // __grid_constant__ parameter, TF staged in shared memory) and the batch
 // kernel (a job table in global memory, chunks of all jobs in one counter).
@@ -1247,6 +1358,7 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
   float3 &shadowFrag = EXT ? shadowFragStore : hitRGB;
   bool shadowRay = false;
   unsigned steps = 0;
+  float draw = 0.f;  // the free-flight draw of a lane in LP_SAMPLE
   // EXT (the instantiation for multi-scatter paths and principled volumes;
   // the plain kernels compile neither): the path's throughput, rounded to binary16 like
   // PathState::throughput (Ray.h:17-23); the MIS weight of the path ray; its
@@ -1619,26 +1731,27 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       }
       const int n = __popc(need);
       const int take = min(n, chunkLeft);
+      bool culled = false;
       const int rank = __popc(need & ((1u << lane) - 1u));
       if (((need >> lane) & 1u) && rank < take) {
         const FrameDD &fr = jobs[chunkJob].fr;
-        const int W = fr.width, H = fr.height;
-        // pixel order: 4-row bands, column-major inside a band (8x4 tiles per 32 pixels)
-        const int w = chunkBase + rank;
-        const int band = w / (4 * W);
-        const int rows = min(4, H - 4 * band);
-        const int within = w - band * 4 * W;
         job = chunkJob;
-        ix = within / rows;
-        iy = 4 * band + within % rows;
-        const int64_t pix = (int64_t)iy * W + ix;
-        k = 0;
-        const bool pixIn = BNB_IN(pix, (long long)fr.width * fr.height);
-        acc = (fr.accumID0 > 0 && pixIn) ? fr.accum[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
-        comp = (CMP && fr.accumID0 > 0 && (CMP == 2 || fr.comp) && pixIn) ? fr.comp[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
-        phase = LP_NEWSAMPLE;
+        chunkPixel(fr, chunkBase + rank, ix, iy);
+        if (pixelMisses(fr, ix, iy)) {  // stays without a pixel
+          missPixel(fr, ix, iy);
+          culled = true;
+        } else {
+          const int64_t pix = (int64_t)iy * fr.width + ix;
+          k = 0;
+          const bool pixIn = BNB_IN(pix, (long long)fr.width * fr.height);
+          acc = (fr.accumID0 > 0 && pixIn) ? fr.accum[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+          comp = (CMP && fr.accumID0 > 0 && (CMP == 2 || fr.comp) && pixIn) ? fr.comp[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+          phase = LP_NEWSAMPLE;
+        }
       }
-      for (int i = 0; i < take; i++) need &= need - 1u;
+      need = __ballot_sync(FULL, phase == LP_IDLE);
+      const int nCulled = __popc(__ballot_sync(FULL, culled));
+      if (nCulled && lane == 0) atomicAdd(&ctr->rays, (unsigned long long)nCulled * (unsigned)jobs[chunkJob].fr.spp);
       chunkBase += take;
       chunkLeft -= take;
     }
@@ -1710,43 +1823,23 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       const FrameDD &fr = J.fr;
       while (true) {
         // ------------------------------------------------------------------
-        // B1. next macrocell with a non-zero majorant (DDA.h:172-200,
-        //    MCAccelerator.h:596-612)
+        // B1. one macrocell of every walking ray
         // ------------------------------------------------------------------
-        if (phase == LP_CELL) {
-          while (true) {
-            const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-            // cell indices are inside the grid here and the grid has < 2^31 cells
-            const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
-            const bool occupied = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z) &&
-                                  ((__ldg(v.mcOccupied + (ci >> 5)) >> (ci & 31)) & 1u);
-            nVisits++;
-            if (!occupied) {  // majorant == 0
-              if (!ddaStep(v, ts, tClosest)) { phase = LP_ENDED; break; }
-              if (++steps > (1u << 22)) { errBits |= ERR_ITER_CAP; phase = LP_ENDED; break; }
-            } else {
-              // no collision can precede a surface hit at or before this cell's start
-              if (ISO && (ts.bits & 64) && ts.rayT0 + ts.nextCellBegin >= ts.rayTMax) { phase = LP_ENDED; break; }
-              ts.maj = __ldg(v.majorants + ci);
-              ts.t = ts.rayT0 + ts.nextCellBegin;
-              ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
-              phase = LP_WOODCOCK;
-              break;
-            }
-          }
-        }
+        const bool exact = LOG == 1 || (LOG == 2 && fr.exactLog);
+        if ((phase == LP_CELL || phase == LP_WOODCOCK) && walkCell<ISO>(v, exact, ts, phase, draw, steps, nVisits))
+          errBits |= ERR_ITER_CAP;
+        const int nWalking = __popc(__ballot_sync(FULL, phase == LP_CELL));
+        if (nWalking > 32 - sd.sampleBatch) continue;
         // ------------------------------------------------------------------
-        // B2. one Woodcock step (Volume.h:180-201)
+        // B2. the steps that end inside their macrocell (Volume.h:180-201):
+        //     sampled together by all lanes that got here since the last time
         // ------------------------------------------------------------------
-        if (phase == LP_WOODCOCK) {
-          const float r = rngFloat(ts.rng);
-          const bool exact = LOG == 1 || (LOG == 2 && fr.exactLog);
-          const float dt = exact ? (-logPortable(1.f - r) / ts.maj) : (-fastLog(1.f - r) / ts.maj);
-          ts.t += dt;
-          if (ts.t >= ts.tUpper) {
-            const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-            phase = ddaStep(v, ts, tClosest) ? LP_CELL : LP_ENDED;
+        if (phase == LP_SAMPLE) {
+          ts.t += exact ? (-logPortable(1.f - draw) / ts.maj) : (-fastLog(1.f - draw) / ts.maj);
+          if (ts.t >= ts.tUpper) {  // (the margin's few)
+            phase = leaveCell(v, ts, fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z)) ? LP_CELL : LP_ENDED;
           } else {
+            phase = LP_WOODCOCK;
             const float3 P = f3(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z);
             const float s = sampleJob<T>(v, P, u8lut);
             nSamples++;
@@ -1776,7 +1869,7 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
               phase = LP_HIT;
             }
           }
-          if (++steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
+          if (steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
             errBits |= ERR_ITER_CAP;
             phase = LP_ENDED;
           }
@@ -1899,16 +1992,6 @@ DEV void ringFetch(float4 *shared, const float4 *p) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(p) : "memory");
 }
 DEV void ringFetchWait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// The pixel's rays cannot meet the volume's bounds: its square lies beyond an
-// edge of their projection (cullEdges in bn_api.cpp, with its error margin).
-DEV bool pixelMisses(const FrameDD &fr, int ix, int iy) {
-  const float x = ix + .5f, y = iy + .5f;
-  bool out = false;
-#pragma unroll
-  for (int e = 0; e < kCullEdges; e++) out = out || fr.cull[e].x * x + fr.cull[e].y * y + fr.cull[e].z > 0.f;
-  return out;
-}
 
 // Path i of a slot with n = popc(mask) issuing pixels is wave i / n: i < 64 and
 // n <= 32, so i ceil(2^16 / n) / 2^16 (error below 64/2^16 < 1/32) is exact.
@@ -2079,29 +2162,6 @@ DEV void retireSlot(const FrameDD &fr, StreamWarp &sw, int s, const float4 *ring
   if (!mine) return;
   fr.accum[pix] = acc;
   if (cmp) fr.comp[pix] = comp;
-}
-
-// True only if the free flight of this draw, RN(-log(1 - draw) / maj), reaches
-// the end of the remaining range `left` whatever its rounding: with the
-// logarithm within 2e-6 of the exact kernels' (a quotient of 2 ulp in a series
-// of one sign), a margin of 1e-5 covers it and the roundings of maj * left.
-// A majorant <= 0 or NaN, a zero draw or an underflowing product give false or
-// a true that holds exactly, so such steps go through the exact evaluation.
-template <int LOG>
-DEV bool leavesCell(float draw, float maj, float left) {
-  float l;
-  if (LOG) {
-    l = -logPortable(1.f - draw);
-  } else {
-    const float u = 1.f - draw;
-    float rcp;  // of a value in [1, 2]: within 1 ulp
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(u + 1.f));
-    const float f = draw * rcp;  // -(u - 1) / (u + 1)
-    const float f2 = f * f;
-    const float s = f + (1.f / 3.f) * (f * f2) + (1.f / 5.f) * (f * f2 * f2);
-    l = s + s;
-  }
-  return maj > 0.f && l * (1.f - 1e-5f) > maj * left;
 }
 
 template <int T, bool BATCH, int LOG>
@@ -2296,44 +2356,10 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
     }
     while (true) {
       // ------------------------------------------------------------------
-      // 6. one macrocell of every walking ray (DDA.h:172-200,
-      //    MCAccelerator.h:596-612): an empty one is left; in one with a
-      //    majorant the free-flight draw of a Woodcock step (Volume.h:180-201)
-      //    is taken.  Most draws leave the macrocell; the distance itself then
-      //    does not matter, so an approximate logarithm decides with a margin,
-      //    and only the draws that may end inside wait for 7, where the exact
-      //    distance is formed.
+      // 6. one macrocell of every walking ray
       // ------------------------------------------------------------------
-      if (phase == LP_CELL || phase == LP_WOODCOCK) {
-        const float tClosest = fmin_(fmin_(ts.tNext.x, ts.tNext.y), ts.tNext.z);
-        bool leaves = false;
-        if (phase == LP_CELL) {
-          // cell indices are inside the grid here and the grid has < 2^31 cells
-          const int ci = ts.cx + v.mcDims.x * (ts.cy + v.mcDims.y * ts.cz);
-          const bool in = BNB_IN(ci, (long long)v.mcDims.x * v.mcDims.y * v.mcDims.z);
-          const float maj = in ? __ldg(v.majorants + ci) : 0.f;
-          leaves = maj == 0.f;
-          nVisits++;
-          if (!leaves) {
-            ts.maj = maj;
-            ts.t = ts.rayT0 + ts.nextCellBegin;
-            ts.tUpper = fmin_(ts.rayT0 + fmin_(tClosest, ts.ddaTMax), ts.rayTMax);
-          }
-        }
-        steps++;
-        if (!leaves) {
-          draw = rngFloat(ts.rng);
-          leaves = leavesCell<LOG>(draw, ts.maj, ts.tUpper - ts.t);
-        }
-        phase = LP_SAMPLE;
-        if (leaves) {
-          phase = leaveCell(v, ts, tClosest) ? LP_CELL : LP_ENDED;
-          if (steps > (1u << 22)) {  // iteration cap: end this ray as if it left the grid
-            atomicOr(&sw.error, ERR_ITER_CAP);
-            phase = LP_ENDED;
-          }
-        }
-      }
+      if ((phase == LP_CELL || phase == LP_WOODCOCK) && walkCell<false>(v, LOG, ts, phase, draw, steps, nVisits))
+        atomicOr(&sw.error, ERR_ITER_CAP);
       const int nWalking = __popc(__ballot_sync(FULL, phase == LP_CELL));
       if (nWalking > 32 - sd.sampleBatch) continue;
       // ------------------------------------------------------------------
@@ -3266,6 +3292,16 @@ cudaError_t launchMapMajorants(const VolumeDD &v, const float2 *ranges, float *m
 }
 #endif  // !BNB_FAST_MATH
 
+// Waiting lanes that end a walking phase, by kernel (ms at 12 / 16 / 20 / 24 / 28):
+// multi-scatter 512^3 10.05 / 10.30 / 10.21 / 10.6 / 11.9 (its tail is pixels'
+// serial waves: latency); isosurface 256^3 8.33 / 8.14 / 8.08 / 7.62 / 7.37 (its
+// ray set-up, the scan, is shared by the lanes that start rays together);
+// streamed 512^3 7.74-7.87 from 18 to 24.
+constexpr int kStreamServiceBatch = 22;
+#ifndef BNB_FAST_MATH
+static int lanesServiceBatch(int ext) { return ext >= 2 ? 28 : ext == 1 ? 12 : 22; }
+#endif
+
 // log2 of the units a 32-pixel chunk is cut into.  A slot holds 64 paths of one
 // unit: fewer pixels with more waves, or more with fewer.  Larger units retire
 // with fewer idle lanes; smaller ones spread a small frame over more warps.
@@ -3303,6 +3339,7 @@ static cudaError_t launchStreamT(const VolumeDD &v, const FrameDD &fr, SchedDD s
   int blocks = 0;
   const cudaError_t e = streamGrid(kern, bps, tpb, smem, ring, blocks);
   if (e != cudaSuccess) return e;
+  if (sd.serviceBatch <= 0) sd.serviceBatch = kStreamServiceBatch;
   sd.unitSplit = unitSplitFor(((long long)fr.width * fr.height + kChunk - 1) / kChunk, fr.spp, blocks * (tpb / 32));
   JobDD job;
   job.v = v;
@@ -3315,11 +3352,12 @@ static cudaError_t launchStreamT(const VolumeDD &v, const FrameDD &fr, SchedDD s
 // The lane-owned kernels: extended jobs, and plain ones on the path that has
 // no ring memory (the no-allocation entry point, without compensated sums).
 template <int T>
-static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, const SchedDD &sd, LaunchCounters *ctr,
+static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, SchedDD sd, LaunchCounters *ctr,
                                 int bps, int tpb, cudaStream_t s) {
   const size_t smem = (size_t)v.tfN * sizeof(float4);
   const bool pvms = fr.maxVolumeBounces > 0 || v.pv.enabled;
   const int ext = v.iso.enabled ? (pvms ? 2 : 3) : pvms ? 1 : 0;
+  if (sd.serviceBatch <= 0) sd.serviceBatch = lanesServiceBatch(ext);
   // kernels with and without compensated sums
   const bool cmp = fr.comp != nullptr;
   if (ext == 0 && cmp) return cudaErrorInvalidValue;
@@ -3447,6 +3485,7 @@ cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkS
   int blocks = 0;
   const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
   if (e != cudaSuccess) return e;
+  if (sd.serviceBatch <= 0) sd.serviceBatch = kStreamServiceBatch;
   sd.unitSplit = unitSplitFor(hostChunkStart[numJobs], 8, blocks * (tpb / 32));
   // host staging of the 31 KB parameter (the launch copies it); one launch
   // at a time fills it
@@ -3473,6 +3512,7 @@ cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJ
     int blocks = 0;
   const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
     if (e != cudaSuccess) return e;
+    if (sd.serviceBatch <= 0) sd.serviceBatch = kStreamServiceBatch;
     sd.unitSplit = unitSplitFor(numChunks, 8, blocks * (tpb / 32));
     kern<<<blocks, tpb, 0, s>>>(jobs, chunkStart, numJobs, sd, ctr, ring.ptr);
     return cudaGetLastError();
@@ -3480,6 +3520,7 @@ cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJ
 #ifdef BNB_FAST_MATH
   return cudaErrorInvalidValue;  // the fast-math object holds the plain kernels only
 #else
+  if (sd.serviceBatch <= 0) sd.serviceBatch = lanesServiceBatch(extended);
   auto kern = extended == 3 && !compensated ? batchKernelFor<3, 0>(voxelType)
               : extended >= 2 ? (compensated ? batchKernelFor<2, 1>(voxelType) : batchKernelFor<2, 0>(voxelType))
                               : (compensated ? batchKernelFor<1, 1>(voxelType) : batchKernelFor<1, 0>(voxelType));
