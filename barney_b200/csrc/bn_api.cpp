@@ -621,6 +621,13 @@ BN_API void bnContextDestroy(BNContext context) {
     owned = std::move(g_contexts[c]);
     g_contexts.erase(c);
   }
+  owned.reset();
+  bool last;
+  {
+    std::lock_guard<std::mutex> l(g_ctxMutex);
+    last = g_contexts.empty();
+  }
+  if (last) deviceBlockCache().flush();
   BN_CATCH()
 }
 

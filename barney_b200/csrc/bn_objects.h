@@ -27,6 +27,7 @@
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
+#include <deque>
 #include <vector>
 
 namespace bnb {
@@ -50,7 +51,70 @@ inline std::atomic<int> &allocFailCountdown() {
   static std::atomic<int> c{-1};
   return c;
 }
-// cudaMalloc, or the injected failure
+// Freed device blocks kept for the next allocation of their size class: a
+// client that opens volume after volume of one size (time steps, a browser of
+// scans) otherwise pays cudaMalloc and cudaFree of every buffer, 2 of the
+// 3.7 ms that opening a 512 MB volume took.  At most kMaxHeld bytes are held
+// (the oldest go first), all of them are freed when an allocation fails and
+// when the last context is destroyed.  A block is entered only once its
+// device is idle, as cudaFree waits for it, so it can be handed to any stream.
+struct DeviceBlockCache {
+  static constexpr size_t kMaxHeld = (size_t)4 << 30;
+  struct Block {
+    void *ptr;
+    size_t bytes;
+    int device;
+  };
+  std::mutex m;
+  std::deque<Block> blocks;
+  size_t held = 0;
+  // cudaMalloc's own granularity: 2 MiB, 512 B below 1 MiB
+  static size_t sizeClass(size_t n) {
+    const size_t g = n < ((size_t)1 << 20) ? 512 : (size_t)2 << 20;
+    return (n + g - 1) / g * g;
+  }
+  void *take(size_t n, int device) {
+    std::lock_guard<std::mutex> l(m);
+    for (auto it = blocks.begin(); it != blocks.end(); ++it)
+      if (it->bytes == n && it->device == device) {
+        void *p = it->ptr;
+        held -= n;
+        blocks.erase(it);
+        return p;
+      }
+    return nullptr;
+  }
+  void put(void *p, size_t n, int device) {
+    std::vector<void *> drop;
+    {
+      std::lock_guard<std::mutex> l(m);
+      blocks.push_back({p, n, device});
+      held += n;
+      while (held > kMaxHeld) {
+        drop.push_back(blocks.front().ptr);
+        held -= blocks.front().bytes;
+        blocks.pop_front();
+      }
+    }
+    for (void *d : drop)
+      if (cudaFree(d) != cudaSuccess) cudaGetLastError();
+  }
+  void flush() {
+    std::deque<Block> all;
+    {
+      std::lock_guard<std::mutex> l(m);
+      all.swap(blocks);
+      held = 0;
+    }
+    for (auto &b : all)
+      if (cudaFree(b.ptr) != cudaSuccess) cudaGetLastError();
+  }
+};
+inline DeviceBlockCache &deviceBlockCache() {
+  static DeviceBlockCache *c = new DeviceBlockCache;  // never destroyed: buffers may be freed at exit
+  return *c;
+}
+// Device memory of the current device, or the injected failure; freed with deviceFree.
 inline cudaError_t deviceMalloc(void **p, size_t n) {
   int c = allocFailCountdown().load();
   while (c >= 0) {
@@ -59,7 +123,29 @@ inline cudaError_t deviceMalloc(void **p, size_t n) {
       break;
     }
   }
-  return cudaMalloc(p, n);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const size_t size = DeviceBlockCache::sizeClass(n);
+  if ((*p = deviceBlockCache().take(size, dev))) return cudaSuccess;
+  e = cudaMalloc(p, size);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  deviceBlockCache().flush();
+  return cudaMalloc(p, size);
+}
+// n: the size deviceMalloc was asked for.
+inline void deviceFree(void *p, size_t n) {
+  if (!p) return;
+  int dev = 0;
+  cudaPointerAttributes at{};
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.device == dev &&
+      DeviceBlockCache::sizeClass(n) <= DeviceBlockCache::kMaxHeld && cudaDeviceSynchronize() == cudaSuccess) {
+    deviceBlockCache().put(p, DeviceBlockCache::sizeClass(n), dev);
+    return;
+  }
+  cudaGetLastError();
+  if (cudaFree(p) != cudaSuccess) cudaGetLastError();
 }
 
 inline void ck(cudaError_t e, const char *what) {
@@ -89,7 +175,7 @@ struct DeviceBuffer {
   DeviceBuffer &operator=(const DeviceBuffer &) = delete;
   ~DeviceBuffer() { release(); }
   void release() {
-    if (ptr && cudaFree(ptr) != cudaSuccess) cudaGetLastError();
+    deviceFree(ptr, bytes);
     ptr = nullptr;
     bytes = 0;
   }
@@ -472,8 +558,8 @@ struct Context {
     if (hostCounters) cudaFreeHost(hostCounters);
     handles.clear();
     for (auto &e : ev) if (e) cudaEventDestroy(e);
-    if (dCounters) cudaFree(dCounters);
-    if (ring.ptr) cudaFree(ring.ptr);
+    deviceFree(dCounters, sizeof(LaunchCounters));
+    deviceFree(ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4));
     if (ownStream) cudaStreamDestroy(ownStream);
     cudaGetLastError();  // nothing of a destroyed context may leak into later calls
   }

@@ -67,7 +67,7 @@ struct BufferPool {
   std::vector<Chunk> chunks;
   size_t deviceBytesHeld = 0;
   ~BufferPool() {
-    for (auto &c : chunks) cudaFree(c.base);
+    for (auto &c : chunks) deviceFree(c.base, c.size);
   }
   void *getDevice(size_t n) {
     const size_t need = (n + 255) & ~(size_t)255;
