@@ -2025,12 +2025,13 @@ __global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2 ? kRenderMinBlocks
 // host) issue no paths; they add their miss colour where they are found (three
 // quarters of the 1080p frame around a cube).
 //
-// Bound: instruction issue and fetch.  Against the lane-owned loop on the 512^3
-// 1080p 64-spp frame (ncu on 8 spp): warp instructions 1.65 -> 1.05 G, 11.1 -> 16.8
-// of 32 lanes a instruction, 14.5 -> 10.0 ms; 256^2 x 16 spp of a 64^3 volume, where
-// a pixel's waves no longer wait for one another, 1.0 -> 0.24 ms; 64 mixed jobs
-// 41 -> 29 ms.  Shading at once in every pass that waits on samples: the steps
-// that end inside a macrocell wait for one another too (4 -> 14 lanes a sample).
+// Bound: instruction issue and fetch (65 % of issue slots, no-instruction stalls
+// 1.7 per issue).  Against the lane-owned loop on the 512^3 1080p 64-spp frame (ncu
+// on 8 spp): warp instructions 1.65 -> 0.84 G, 11.1 -> 19.3 of 32 lanes an
+// instruction, kernel 14.5 -> 7.8 ms; 256^2 x 16 spp of a 64^3 volume, where a
+// pixel's waves no longer wait for one another, 1.0 -> 0.22 ms; 64 mixed jobs
+// 41 -> 24 ms.  Steps that end inside a macrocell wait for one another too: 4 -> 20
+// lanes a sample.
 constexpr float kPathOccluded = 0.f, kPathLit = 1.f, kPathMissed = 2.f;  // outcome in the ring entry's w
 
 // A warp's shared memory: everything its lanes do not need between two

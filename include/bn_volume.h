@@ -311,7 +311,8 @@ BN_API void bnxSetRegrouping(BNContext context, int enable);
 /* Warp scheduling of the render kernel: a warp keeps stepping macrocells and
    Woodcock ranges until at least serviceBatch of its lanes (or all of its
    busy lanes) need service -- shading, accumulation, a new ray -- and then
-   serves them together (1..32, default 22). */
+   serves them together (1..32; until it is set, each kernel's own default:
+   22 plain, 12 multi-scatter, 28 isosurface). */
 BN_API void bnxSetScheduling(BNContext context, int serviceBatch);
 /* Bounds-checked build (libbarney_b200_bc.so, python -m barney_b200.build
    --bounds-check): every indexed access of the render and macrocell kernels
