@@ -2193,10 +2193,11 @@ DEV void retireSlot(const FrameDD &fr, StreamWarp &sw, int s, const float4 *ring
   float4 comp = mine && cmp && accumID > 0 ? fr.comp[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 bg = missColor(fr, iy);
   const bool issues = (m >> lane) & 1u;
-  // a pixel that issues no paths, with a miss that adds alpha 1 and no colour:
-  // whole numbers below 2^24 add without rounding, so its waves are one
-  // addition (which leaves the compensation terms as they are)
-  const bool whole = !issues && bg.w == 1.f && !(bg.x > 0.f) && !(bg.y > 0.f) && !(bg.z > 0.f) && accumID > 0 &&
+  // a pixel that issues no paths, with a miss that adds alpha 1 and no colour
+  // (a NaN component does: the clamp turns it into clampMax): whole numbers
+  // below 2^24 add without rounding, so its waves are one addition (which
+  // leaves the compensation terms as they are)
+  const bool whole = !issues && bg.w == 1.f && bg.x <= 0.f && bg.y <= 0.f && bg.z <= 0.f && accumID > 0 &&
                      acc.w >= 0.f && acc.w == truncf(acc.w) && acc.w <= 8388608.f && waves <= 8388608;
   if (whole) acc.w += (float)waves;
   if (!mine || whole) waves = 0;

@@ -38,9 +38,11 @@ def test_wide_frame(spp):
 
 
 # what a pixel outside the volume adds: black with alpha 1 (one addition),
-# colours, alpha that rounds, a gradient per row, colours above the clamp
+# colours, alpha that rounds, a gradient per row, colours above the clamp, NaN
+# (the clamp's value)
 @pytest.mark.parametrize("bg", [(0.0, 0.0, 0.0, 1.0), (0.2, 0.0, 0.7, 1.0), (0.0, 0.0, 0.0, 0.3), (0.1, 0.2, 0.3, -1.0),
-                                (25.0, 0.0, 3.0, 1.0), (-0.5, 0.0, -0.0, 0.0)])
+                                (25.0, 0.0, 3.0, 1.0), (-0.5, 0.0, -0.0, 0.0), (np.nan, 0.0, -1.0, 1.0),
+                                (0.0, -np.inf, np.nan, 1.0)])
 @pytest.mark.parametrize("comp", [False, True])
 def test_pixels_outside_the_volume(bg, comp):
     d = small_noise_scene(n=20, w=70, h=41, bg_color=bg, compensated_accum=comp, majorant_round_up=comp,
