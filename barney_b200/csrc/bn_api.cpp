@@ -465,7 +465,8 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
   reserveBatch(ctx, n);
   std::vector<const void *> key;
   long long chunks = 0;
-  unsigned long long pixelSamples = 0;
+  unsigned long long pixelSamples = 0, chunkWaves = 0;
+  double sppSum = 0.;  // of each path's job
   int extended = 0;  // 1: multi-scatter, principled or exact log; 2: isosurfaces (the extended kernels)
   bool anyIso = false, anyPvms = false;
   int voxelType = -2;     // the type every job shares, else -1
@@ -484,10 +485,14 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
     fast = fast && job.fr.fastMath;
     compJobs += job.fr.comp != nullptr;
     ctx->hostJobs[i] = job;
-    chunks += ((long long)job.fr.width * job.fr.height + 31) / 32;
+    const long long jobChunks = ((long long)job.fr.width * job.fr.height + 31) / 32;
+    chunks += jobChunks;
     if (chunks > 0x7fffffffLL) throw Error(E_INVALID_ARG, "batch too large");
     ctx->hostChunks[i + 1] = (int)chunks;
-    pixelSamples += (unsigned long long)job.fr.width * job.fr.height * job.fr.spp;
+    const unsigned long long paths = (unsigned long long)job.fr.width * job.fr.height * job.fr.spp;
+    pixelSamples += paths;
+    sppSum += (double)paths * job.fr.spp;
+    chunkWaves += (unsigned long long)jobChunks * job.fr.spp;
     key.push_back(e.fb);
     key.push_back(e.fb->accum.ptr);
     key.push_back(e.fb->comp.ptr);
@@ -496,6 +501,8 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
   key.push_back((const void *)(intptr_t)(ctx->blocksPerSM * 4096 + ctx->threadsPerBlock));
   key.push_back((const void *)(intptr_t)ctx->sched.serviceBatch);
   key.push_back((const void *)(intptr_t)n);
+  const int spp = (int)std::min(sppSum / (double)pixelSamples, 1e9);
+  key.push_back((const void *)(intptr_t)std::min(spp, 8));  // the unit size is captured (unitSplitFor)
   // isosurfaces without volume bounces or principled volumes: the smaller kernel
   if (anyIso && !anyPvms) extended = 3;
   key.push_back((const void *)(intptr_t)extended);
@@ -527,14 +534,14 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
        "chunk table");
     ck(cudaMemsetAsync(ctx->dCounters, 0, sizeof(LaunchCounters), s), "counter reset");
     if (timed) ck(cudaEventRecord(ctx->ev[0], s), "event");
-    if (!ctx->useGraphs && extended == 0 && n <= kParamJobs)  // the jobs as one kernel parameter
+    if (!ctx->useGraphs && extended == 0 && batchAsParams(n, chunkWaves))  // the jobs as one kernel parameter
       ck((fast ? fastmath::launchRenderBatchParams : launchRenderBatchParams)(
-             ctx->hostJobs, ctx->hostChunks, n, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
+             ctx->hostJobs, ctx->hostChunks, n, spp, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
              voxelType, ctx->ring),
          "batch render kernel");
     else
       ck((fast ? fastmath::launchRenderBatch : launchRenderBatch)(
-             (const JobDD *)ctx->batchJobs.ptr, (const int *)ctx->batchChunks.ptr, n, (int)chunks, ctx->dCounters,
+             (const JobDD *)ctx->batchJobs.ptr, (const int *)ctx->batchChunks.ptr, n, (int)chunks, spp, ctx->dCounters,
              ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched, extended, voxelType, compJobs > 0, ctx->ring),
          "batch render kernel");
     if (timed) ck(cudaEventRecord(ctx->ev[1], s), "event");

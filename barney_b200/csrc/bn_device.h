@@ -157,7 +157,8 @@ cudaError_t launchMapMajorants(const VolumeDD &vol, const float2 *ranges, float 
 cudaError_t launchRender(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, int blocksPerSM,
                          int threadsPerBlock, cudaStream_t s, const SchedDD &sd, const StreamRing &ring);
 // jobs / chunkStart: device arrays; chunkStart has numJobs+1 entries, the
-// prefix sum of each job's ceil(width*height/32) pixel chunks, numChunks in all.
+// prefix sum of each job's ceil(width*height/32) pixel chunks, numChunks in all;
+// spp: the waves of a path's job, averaged over the launch's paths.
 // extended: 2 if some job has an isosurface and some job volume bounces
 // (fr.maxVolumeBounces > 0) or a principled volume, 3 if some job has an
 // isosurface and none has either, else 1 if some job has volume bounces, a
@@ -165,16 +166,18 @@ cudaError_t launchRender(const VolumeDD &vol, const FrameDD &frame, LaunchCounte
 // instantiation that implements them); voxelType: the
 // VoxelType all jobs share (a kernel compiled for it) or -1 (mixed);
 // compensated (extended kernels): some job carries compensation terms (fr.comp)
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks, int spp,
                               LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
                               SchedDD sd, int extended, int voxelType, int compensated, const StreamRing &ring);
 // The same for at most kParamJobs plain jobs (extended 0) whose table and
 // chunk prefix are in host memory: passed as one kernel parameter.  Not for
-// stream capture (the parameter would be frozen into the graph).
+// stream capture (the parameter would be frozen into the graph).  batchAsParams:
+// whether that is the faster form for a batch with this sum of chunks x waves.
 constexpr int kParamJobs = 31;
+bool batchAsParams(int numJobs, unsigned long long chunkWaves);
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
-                                    LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
-                                    SchedDD sd, int voxelType, const StreamRing &ring);
+                                    int spp, LaunchCounters *counters, int blocksPerSM, int threadsPerBlock,
+                                    cudaStream_t s, SchedDD sd, int voxelType, const StreamRing &ring);
 cudaError_t launchResolve(const float4 *accum, int numPixels, int accumID, int fmt, void *out, cudaStream_t s,
                           const float4 *comp = nullptr);
 // resolves every job of a batch table into its fr.color after its waves
@@ -209,12 +212,12 @@ cudaError_t launchSampleProbe(const VolumeDD &vol, const float3 *P, int n, float
 namespace fastmath {
 cudaError_t launchRender(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, int blocksPerSM,
                          int threadsPerBlock, cudaStream_t s, const SchedDD &sd, const StreamRing &ring);
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks, int spp,
                               LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
                               SchedDD sd, int extended, int voxelType, int compensated, const StreamRing &ring);
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
-                                    LaunchCounters *counters, int blocksPerSM, int threadsPerBlock, cudaStream_t s,
-                                    SchedDD sd, int voxelType, const StreamRing &ring);
+                                    int spp, LaunchCounters *counters, int blocksPerSM, int threadsPerBlock,
+                                    cudaStream_t s, SchedDD sd, int voxelType, const StreamRing &ring);
 cudaError_t launchSampleProbe(const VolumeDD &vol, const float3 *P, int n, float *scalar, float4 *rgba, cudaStream_t s);
 cudaError_t launchRenderRegrouped(const VolumeDD &vol, const FrameDD &frame, LaunchCounters *counters, cudaStream_t s);
 long long readBoundsViolationsHere();  // bounds-checked build only

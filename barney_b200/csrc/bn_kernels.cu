@@ -3378,16 +3378,26 @@ constexpr int kStreamServiceBatch = 22;
 static int lanesServiceBatch(int ext) { return ext >= 2 ? 28 : ext == 1 ? 12 : 22; }
 #endif
 
-// log2 of the units a 32-pixel chunk is cut into.  A slot holds 64 paths of one
-// unit: fewer pixels with more waves, or more with fewer.  Larger units retire
+// log2 of the units a 32-pixel chunk is cut into.  A slot holds at most 64 paths of
+// one unit: fewer pixels with more waves, or more with fewer.  Larger units retire
 // with fewer idle lanes; smaller ones spread a small frame over more warps.
-// Measured (kernel ms at 32 / 16 / 8 pixels a unit): 512^3 1080p 64 spp 7.86 /
-// 7.78 / 8.08; 1024^2 4 spp 0.496 / 0.515 / 0.610; 1279x719 1 spp 0.134 / 0.196 /
-// 0.331 (slots of 32, 16 and 8 paths); 256^2 16 spp, 2048 chunks over 4144 warps,
-// 0.499 / 0.351 / 0.217.
+// chunks: of the whole launch; spp: a path's frame's waves, averaged over the paths.
+// Measured (kernel ms at 32 / 16 / 8 pixels a unit, 4144 warps):
+//   chunks  frames          1 spp              2 spp              4 spp              16 spp
+//     2048  256^2           .051 .052 .060     .068 .057 .066     .104 .083 .075     .344 .230 .160
+//     8192  512^2           .075 .092 .132     .101 .109 .142     .156 .156 .172     .501 .481 .470
+//    16384  8 x 256^2       .160 .187 .265     .219 .222 .281     .346 .342 .367     1.14 1.04 1.08
+//    32768  1024^2          .217 .278 .417     .327 .360 .476     .552 .562 .661     1.95 1.89 1.94
+//    64800  1080p, 64 spp   7.86 7.78 8.08
+//   131072  64 x 256^2      .724 .909 1.38     1.17 1.30 1.64     2.09 2.19 2.52     7.48 7.57 8.00
+// (8 x 256^2 and up are batches.)  A launch of a pixel partition counts the whole
+// frame's chunks: its share of 1080p on 8 ranks takes .179 / .300 / 1.055 ms at 8 / 16 /
+// 64 spp so, and .185 / .306 / 1.030 with the share's own count.
 static int unitSplitFor(long long chunks, int spp, int warps) {
-  if (spp < 8) return 0;
-  return chunks < 4LL * warps ? 2 : 1;
+  if (spp >= 8) return chunks < 4LL * warps ? 2 : 1;
+  if (spp >= 4) return chunks < warps ? 2 : chunks < 6LL * warps ? 1 : 0;
+  if (spp >= 2) return 2 * chunks < 3LL * warps ? 1 : 0;
+  return 0;
 }
 
 // Blocks of a launch: bps per SM (0: as many as fit), at most the warps that
@@ -3547,9 +3557,25 @@ __global__ void __launch_bounds__(kRenderMaxThreads, kRenderMinBlocks)
   streamLoop<T, true, 0>(tab.jobs, tab.chunkStart, numJobs, tab.chunkStart[numJobs], sd, ctr, streamRing(ring),
                          sWarp[threadIdx.x >> 5], nullptr, u8lut);
 }
+#ifndef BNB_FAST_MATH
+// A lane reads its own job's fields.  In the constant bank lanes of one job share a
+// read and lanes of different jobs take turns; a table in global memory is slower for
+// one job and does not care.  Paths of several jobs meet in a warp while a job is small
+// against the launch's warps.  Measured (kernel ms, parameter / table, 4144 warps; a
+// job's chunks x spp in brackets):
+//    4 jobs  256^2 16 spp .544 / .559    512^2 1 spp .209 / .189 [8 K]    4 spp .526 / .525
+//    8 jobs  256^2 1 spp .172 / .131 [2 K]   16 spp 1.062 / 1.057 [33 K]   64 spp 3.64 / 3.82 [131 K]
+//            512^2 1 spp .440 / .323 [8 K]    4 spp  .995 /  .980 [33 K]    8 spp 1.83 / 1.89 [66 K]
+//   31 jobs  128^2 8 spp 1.20 / .604 [4 K]   256^2 1 spp .879 / .347 [2 K]  16 spp 4.05 / 3.74 [33 K]
+//            512^2 1 spp 1.95 / 1.15 [8 K]    4 spp 3.77 / 3.64 [33 K]      8 spp 6.96 / 7.18 [66 K]
+bool batchAsParams(int numJobs, unsigned long long chunkWaves) {
+  if (numJobs > kParamJobs) return false;
+  return numJobs <= 4 || chunkWaves >= 10ull * kRenderMinBlocks * (kRenderMaxThreads / 32) * smCount() * numJobs;
+}
+#endif
 cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkStart, int numJobs,
-                                    LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd, int voxelType,
-                                    const StreamRing &ring) {
+                                    int spp, LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd,
+                                    int voxelType, const StreamRing &ring) {
   if (numJobs < 1 || numJobs > kParamJobs) return cudaErrorInvalidValue;
   if (tpb <= 0) tpb = 128;
   auto kern = voxelType == VOX_F32    ? streamBatchParamKernel<VOX_F32>
@@ -3562,7 +3588,7 @@ cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkS
   const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
   if (e != cudaSuccess) return e;
   if (sd.serviceBatch <= 0) sd.serviceBatch = kStreamServiceBatch;
-  sd.unitSplit = unitSplitFor(hostChunkStart[numJobs], 8, blocks * (tpb / 32));
+  sd.unitSplit = unitSplitFor(hostChunkStart[numJobs], spp, blocks * (tpb / 32));
   // host staging of the 31 KB parameter (the launch copies it); one launch
   // at a time fills it
   static JobTableParam tab;
@@ -3574,9 +3600,9 @@ cudaError_t launchRenderBatchParams(const JobDD *hostJobs, const int *hostChunkS
   return cudaGetLastError();
 }
 
-cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks,
-                              LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd, int extended, int voxelType, int compensated,
-                              const StreamRing &ring) {
+cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJobs, int numChunks, int spp,
+                              LaunchCounters *ctr, int bps, int tpb, cudaStream_t s, SchedDD sd, int extended,
+                              int voxelType, int compensated, const StreamRing &ring) {
   if (tpb <= 0) tpb = 128;
   if (!extended) {
     auto kern = voxelType == VOX_F32    ? streamBatchKernel<VOX_F32>
@@ -3586,10 +3612,10 @@ cudaError_t launchRenderBatch(const JobDD *jobs, const int *chunkStart, int numJ
                 : voxelType == VOX_BF16 ? streamBatchKernel<VOX_BF16>
                                         : streamBatchKernel<-1>;
     int blocks = 0;
-  const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
+    const cudaError_t e = streamGrid(kern, bps, tpb, 0, ring, blocks);
     if (e != cudaSuccess) return e;
     if (sd.serviceBatch <= 0) sd.serviceBatch = kStreamServiceBatch;
-    sd.unitSplit = unitSplitFor(numChunks, 8, blocks * (tpb / 32));
+    sd.unitSplit = unitSplitFor(numChunks, spp, blocks * (tpb / 32));
     kern<<<blocks, tpb, 0, s>>>(jobs, chunkStart, numJobs, sd, ctr, ring.ptr);
     return cudaGetLastError();
   }

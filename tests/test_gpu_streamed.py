@@ -24,15 +24,15 @@ def check(d, spp, what, renders=1):
     assert st["error_flags"] == 0
 
 
-# spp 1-3: 32 pixels a unit; 4-7: 16; from 8 on 8 pixels and 8 waves a slot on small frames
+# small frames: 32 pixels a unit at 1 spp, 16 at 2-3, 8 from 4 on (8 waves a slot from 8 on)
 @pytest.mark.parametrize("size", [(1, 1), (7, 1), (8, 4), (9, 5), (33, 31), (31, 66)])
 @pytest.mark.parametrize("spp", [1, 2, 3, 4, 7, 8, 9, 17, 64, 65])
 def test_units_and_slots(size, spp):
     check(small_noise_scene(n=24, w=size[0], h=size[1], camera=synth.look_at((1.1, 0.9, 1.2))), spp, f"{size} {spp}")
 
 
-# a frame wide enough that units of 16 pixels and many slots are in flight
-@pytest.mark.parametrize("spp", [8, 33])
+# a frame wide enough that units of 32 (2 spp) and 16 pixels and many slots are in flight
+@pytest.mark.parametrize("spp", [2, 5, 8, 33])
 def test_wide_frame(spp):
     check(small_blob_scene(n=20, w=1021, h=563), spp, f"wide {spp}")
 
@@ -82,3 +82,65 @@ def test_emission_absorption_over_renders():
     d = small_blob_scene(n=20, w=37, h=29, emission_absorption=True, ambient=0.0)
     check(d, 9, "emission-absorption")
     check(d, 4, "emission-absorption, three renders", renders=3)
+
+
+# Batches: lanes of a warp hold paths of several jobs.  The jobs differ in storage,
+# size, sums, background and camera; some see nothing of their volume.
+def batch_scenes(n):
+    out = []
+    for i in range(n):
+        kw = {"camera": synth.look_at((4.0, 3.0, 4.0) if i % 7 == 5 else (1.1, 0.9, 1.2) if i % 3 else (2.0, 1.5, 2.0),
+                                      target=(9.0, 9.0, 9.0) if i % 7 == 3 else synth.CUBE_CENTRE)}
+        if i % 4 == 1:
+            kw.update(compensated_accum=True, majorant_round_up=True)
+        if i % 5 == 2:
+            kw["bg_color"] = (0.2, 0.0, 0.7, 1.0)
+        w, h = [(33, 31), (7, 1), (9, 5), (31, 66), (64, 24)][i % 5]
+        out.append(small_noise_scene(n=[24, 13, 20][i % 3], w=w, h=h, dtype=["f32", "u8", "f16"][i % 3], **kw))
+    return out
+
+
+def check_batch(scenes, spps, graphs, renders):
+    import barney_b200 as bn
+    ctx = bn.Context()
+    ctx.set_graphs(graphs)
+    rs = [bn.VolumeRenderer(d, context=ctx) for d in scenes]
+    for r, spp in zip(rs, spps):
+        r.set_spp(spp)
+    for _ in range(renders):
+        ctx.render_batch(rs)
+    assert ctx.stats()["error_flags"] == 0
+    for i, (r, d, spp) in enumerate(zip(rs, scenes, spps)):
+        acc = np.zeros((d["height"], d["width"], 4), np.float32)
+        comp = np.zeros_like(acc) if d.get("compensated_accum") else None
+        oracle.render(oracle.Scene(d), 0, spp * renders, accum=acc, comp=comp)
+        assert_bitexact(r.read(), oracle.resolve(acc, spp * renders, comp=comp), f"job {i}, {spp} spp")
+        r.close()
+    ctx.close()
+
+
+# at most 4 jobs without graphs travel as a kernel parameter
+@pytest.mark.parametrize("graphs", [False, True])
+@pytest.mark.parametrize("n", [2, 4, 5, 12])
+@pytest.mark.parametrize("spps", [[1], [2], [4], [9], [1, 7, 8, 33, 65]])
+def test_batches(n, spps, graphs):
+    check_batch(batch_scenes(n), [spps[i % len(spps)] for i in range(n)], graphs, 2)
+
+
+# 31 jobs as a parameter and 32 as a table: a large frame beside its volume carries the
+# paths that make the parameter the choice
+@pytest.mark.parametrize("n", [31, 32])
+def test_batches_at_the_parameter_limit(n):
+    scenes = batch_scenes(n - 1)
+    scenes.insert(3, small_noise_scene(n=12, w=1024, h=1024, camera=synth.look_at((2.0, 1.5, 2.0), target=(9.0, 9.0, 9.0))))
+    spps = [[1, 7, 8, 33][i % 4] for i in range(n - 1)]
+    spps.insert(3, 42)
+    check_batch(scenes, spps, False, 1)
+
+
+# enough chunks for units of 16 pixels at 8 spp, and of 32 below
+@pytest.mark.parametrize("spp", [2, 4, 9])
+def test_large_batch(spp):
+    scenes = [small_noise_scene(n=20, w=509, h=601, camera=synth.look_at(p))
+              for p in ((4.0, 3.0, 4.0), (6.0, -3.0, 2.0), (3.0, 9.0, 4.0))]
+    check_batch(scenes, [spp] * 3, False, 1)
