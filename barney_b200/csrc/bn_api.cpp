@@ -174,87 +174,82 @@ static IsoDD isoDD(const IsoSurface &g, const float2 *ranges, const int mcDims[3
 // ---------------------------------------------------------------------------
 // pixels whose rays cannot meet the volume
 // ---------------------------------------------------------------------------
-// Edges of the projection of the field's bounds, in pixels, for
-// FrameDD::cull: a pixel beyond an edge by more than the error margin sends
-// no ray that passes the box test of traceBegin.  The projection of a box in
-// front of the camera is the convex hull of its corners' projections; without
-// that (a corner beside or behind the camera, a cut plane that moves ray
-// origins, non-finite input) no pixel is ruled out.
+// Half-planes of the image that no ray meeting the field's bounds belongs to, for
+// FrameDD::cull.  From a point outside a box the rays that meet it form a convex
+// cone; each of its faces holds an edge of the box, and a ray beyond a face by more
+// than the error margin misses.  Faces are linear in the pixel, so this needs no
+// corner to lie in front of the camera.  No pixel is ruled out from inside the box
+// or close to its surface, by non-finite input, or with a cut plane (it moves ray
+// origins) -- unless that removes the whole box.
 //
-// The margin covers what separates the kernels' binary32 rays from the exact
-// ones: one pixel, plus an angle of 1e-5 (the zero fix-up of a direction's
-// components moves it by at most 1e-6 each; rounding of the direction and of
-// the box test's slab distances is below 2e-6).
+// The margin covers what separates the kernels' binary32 rays from the exact ones:
+// a pixel, plus 2e-5 of the longest unnormalised direction.  The zero fix-up of a
+// direction's components moves it by at most 1e-6 each, rounding of the direction
+// and of the box test's slab distances by less than 2e-6, and a face that passes
+// the corner test below is off by at most 1e-5.
 static void cullEdges(const VolumeDD &v, FrameDD &fr) {
   for (auto &e : fr.cull) e = make_float3(0.f, 0.f, 0.f);
-  if (fr.cutPlane.w > -1e28f) return;
-  const double d0[3] = {fr.dir00.x, fr.dir00.y, fr.dir00.z}, du[3] = {fr.dirdu.x, fr.dirdu.y, fr.dirdu.z},
-               dv[3] = {fr.dirdv.x, fr.dirdv.y, fr.dirdv.z}, o[3] = {fr.lens00.x, fr.lens00.y, fr.lens00.z};
-  // rows of the inverse of [d0 du dv]
-  auto crs = [](const double *a, const double *b, double *r) {
-    r[0] = a[1] * b[2] - a[2] * b[1];
-    r[1] = a[2] * b[0] - a[0] * b[2];
-    r[2] = a[0] * b[1] - a[1] * b[0];
-  };
-  auto dt = [](const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
-  double r0[3], ru[3], rv[3];
-  crs(du, dv, r0);
-  crs(dv, d0, ru);
-  crs(d0, du, rv);
-  const double det = dt(d0, r0);
-  if (!(std::fabs(det) > 1e-12) || !std::isfinite(det)) return;
-  for (int a = 0; a < 3; a++) { r0[a] /= det; ru[a] /= det; rv[a] /= det; }
+  struct d3 { double x, y, z; };
+  auto crs = [](d3 a, d3 b) { return d3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; };
+  auto dt = [](d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; };
+  auto norm = [&](d3 a) { return std::sqrt(dt(a, a)); };
+  auto wide = [](float3 a) { return d3{a.x, a.y, a.z}; };
+  const d3 d0 = wide(fr.dir00), du = wide(fr.dirdu), dv = wide(fr.dirdv), o = wide(fr.lens00);
   const double W = fr.width, H = fr.height, aspect = fr.aspect;
-  // the error of a ray in pixels: an angle of 1e-5 against the longest
-  // unnormalised direction of the image, through the inverse's rows
-  const double su = 0.5 * aspect, sv = 0.5;
-  const double len = std::sqrt(dt(d0, d0)) + su * std::sqrt(dt(du, du)) + sv * std::sqrt(dt(dv, dv));
-  const double n0 = std::sqrt(dt(r0, r0)), nu = std::sqrt(dt(ru, ru)), nv = std::sqrt(dt(rv, rv));
-  const double ex = 1e-5 * len * (nu + 2 * su * n0) / aspect * W, ey = 1e-5 * len * (nv + 2 * sv * n0) * H;
-  double px[8], py[8];
+  const double len = norm(d0) + .5 * aspect * norm(du) + .5 * norm(dv);
+  // (a longer or shorter direction overflows or vanishes when the kernels normalise it)
+  if (!(len > 1e-15 && len < 1e15)) return;
+  d3 q[8];  // the corners, from the camera
+  double qLen[8], qMax = 0., corner = 0.;
   for (int c = 0; c < 8; c++) {
-    const double q[3] = {((c & 1) ? v.boundsHi.x : v.boundsLo.x) - o[0], ((c & 2) ? v.boundsHi.y : v.boundsLo.y) - o[1],
-                         ((c & 4) ? v.boundsHi.z : v.boundsLo.z) - o[2]};
-    const double depth = dt(r0, q);
-    // in front of the camera by a margin against the distance, so that the
-    // projection is well-conditioned
-    if (!(depth > 1e-3 * n0 * std::sqrt(dt(q, q))) || !(depth > 0.0)) return;
-    px[c] = (dt(ru, q) / depth / aspect + 0.5) * W;
-    py[c] = (dt(rv, q) / depth + 0.5) * H;
-    if (!std::isfinite(px[c]) || !std::isfinite(py[c]) || std::fabs(px[c]) > 1e7 || std::fabs(py[c]) > 1e7) return;
+    const d3 p = {(c & 1) ? v.boundsHi.x : v.boundsLo.x, (c & 2) ? v.boundsHi.y : v.boundsLo.y,
+                  (c & 4) ? v.boundsHi.z : v.boundsLo.z};
+    q[c] = {p.x - o.x, p.y - o.y, p.z - o.z};
+    qLen[c] = norm(q[c]);
+    if (!std::isfinite(qLen[c])) return;
+    qMax = std::max(qMax, qLen[c]);
+    corner = std::max(corner, norm(p));
   }
-  // convex hull by gift wrapping from the leftmost corner; an edge of the hull
-  // keeps every corner on its inner side
-  int start = 0;
-  for (int c = 1; c < 8; c++)
-    if (px[c] < px[start] || (px[c] == px[start] && py[c] < py[start])) start = c;
-  int cur = start, edges = 0;
-  do {
-    int next = -1;
+  auto beside = [](double a, double b) { return std::max(0., std::max(std::min(a, b), -std::max(a, b))); };
+  const d3 gap = {beside(q[0].x, q[7].x), beside(q[0].y, q[7].y), beside(q[0].z, q[7].z)};
+  if (!(norm(gap) > 1e-4 * qMax)) return;  // inside, or too close for the margins
+  if (fr.cutPlane.w > -1e28f) {
+    const d3 N = {fr.cutPlane.x, fr.cutPlane.y, fr.cutPlane.z};
+    const double w = fr.cutPlane.w, margin = 1e-3 * (norm(N) * (norm(o) + corner) + std::fabs(w));
+    bool removed = std::isfinite(margin);
+    for (int c = 0; c < 8; c++) removed = removed && dt(N, q[c]) + dt(N, o) + w < -margin;
+    if (removed) fr.cull[0] = make_float3(0.f, 0.f, 1.f);
+    return;
+  }
+  d3 face[kCullEdges];
+  int faces = 0;
+  for (int e = 0; e < 12; e++) {
+    const int axis = 1 << e / 4, other = e % 4;  // edge from corner a along the axis to b
+    const int a = axis == 1 ? 2 * other : axis == 2 ? (other & 1) | (other & 2) << 1 : other, b = a | axis;
+    d3 n = crs(q[a], q[b]);
+    const double l = norm(n);
+    if (!(l > 0.)) continue;
+    n = {n.x / l, n.y / l, n.z / l};
+    bool outer = true, inner = true;  // every corner on n's negative, positive side
     for (int c = 0; c < 8; c++) {
-      if (px[c] == px[cur] && py[c] == py[cur]) continue;
-      if (next < 0) { next = c; continue; }
-      const double t = (px[next] - px[cur]) * (py[c] - py[cur]) - (py[next] - py[cur]) * (px[c] - px[cur]);
-      const auto d2 = [&](int k) { return (px[k] - px[cur]) * (px[k] - px[cur]) + (py[k] - py[cur]) * (py[k] - py[cur]); };
-      if (t < 0 || (t == 0 && d2(c) > d2(next))) next = c;
+      outer = outer && dt(n, q[c]) <= 1e-9 * qLen[c];
+      inner = inner && dt(n, q[c]) >= -1e-9 * qLen[c];
     }
-    if (next < 0) return;  // all corners project to one point
-    // outward normal of the edge cur -> next (corners on its left)
-    double a = py[next] - py[cur], b = -(px[next] - px[cur]);
-    const double l = std::sqrt(a * a + b * b);
-    a /= l;
-    b /= l;
-    double off = -1e300;  // the farthest corner along the normal
-    for (int c = 0; c < 8; c++) off = std::max(off, a * px[c] + b * py[c]);
-    // every point of the pixel's square lies beyond the edge by the margin:
-    // half the square and one pixel along the normal, the ray's error, and
-    // the binary32 rounding of the kernel's test
-    const double margin = 1.5 * (std::fabs(a) + std::fabs(b)) + std::fabs(a) * ex + std::fabs(b) * ey +
-                          1e-6 * (W + H + std::fabs(off));
-    if (edges < kCullEdges) fr.cull[edges] = make_float3((float)a, (float)b, (float)(-off - margin));
-    edges++;
-    cur = next;
-  } while (cur != start && edges < 16);
+    if (!outer && !inner) continue;
+    if (!outer) n = {-n.x, -n.y, -n.z};
+    bool known = faces == kCullEdges;  // a cone of a box has at most six faces
+    for (int f = 0; f < faces; f++) known = known || dt(n, face[f]) > 1. - 1e-9;
+    if (known) continue;
+    face[faces] = n;
+    // n . (d0 + su du + sv dv) as a x + b y + c of the pixel's centre
+    const double px = aspect * dt(n, du) / W, py = dt(n, dv) / H, p0 = dt(n, d0) - .5 * (px * W + py * H);
+    // every ray of the pixel is beyond the face by the margin: half the pixel's
+    // square and one pixel, the ray's error, and the kernel's binary32 rounding
+    const double margin = 1.5 * (std::fabs(px) + std::fabs(py)) + 2e-5 * len +
+                          1e-6 * (std::fabs(px) * W + std::fabs(py) * H + std::fabs(p0));
+    if (std::isfinite(px) && std::isfinite(py) && std::isfinite(p0 - margin))
+      fr.cull[faces++] = make_float3((float)px, (float)py, (float)(p0 - margin));
+  }
 }
 
 // ---------------------------------------------------------------------------

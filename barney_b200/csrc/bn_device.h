@@ -23,7 +23,7 @@ constexpr int kRenderMinBlocksExt = 5;  // extended (multi-scatter, principled):
 constexpr int kRenderMinBlocksIso = 4;  // extended with isosurfaces: 4 x 128 (128; with the warp-cooperative
                                         // iso scan 3 % faster than 5 x 128, which spilled up to 820 B)
 
-constexpr int kCullEdges = 6;           // a box projects to at most a hexagon
+constexpr int kCullEdges = 6;           // the cone of rays that meet a box has at most six faces
 // Streamed render loop: paths of a ring slot, slots of a warp's ring.
 constexpr int kStreamSlotPaths = 64;
 constexpr unsigned kStreamSlots = 16;
@@ -103,8 +103,8 @@ struct FrameDD {
   int partRank, partCount;  // pixel-tile partition: render the tiles t with t % partCount == partRank
   float4 *accum;        // width*height, linear
   float4 *comp;         // width*height Neumaier compensation terms, or null (plain sums)
-  // edges of the volume bounds' projection in pixels: pixel (x, y) with
-  // a (x + .5) + b (y + .5) + c > 0 for some edge sends no ray that meets the
+  // half-planes of the image beside the volume: pixel (x, y) with
+  // a (x + .5) + b (y + .5) + c > 0 for one of them sends no ray that meets the
   // bounds (bn_api.cpp cullEdges; all zero: no pixel is ruled out)
   float3 cull[kCullEdges];
   int accumID0;         // accumID of the first wave of this launch

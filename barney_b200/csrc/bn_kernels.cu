@@ -1348,8 +1348,8 @@ DEV bool shadeVolumeHit(const VolumeDD &v, const FrameDD &fr, float3 P, float tH
   return true;
 }
 
-// The pixel's rays cannot meet the volume's bounds: its square lies beyond an
-// edge of their projection (cullEdges in bn_api.cpp, with its error margin).
+// The pixel's rays cannot meet the volume's bounds: its square lies beyond a face
+// of the cone of rays that do (cullEdges in bn_api.cpp, with its error margin).
 DEV bool pixelMisses(const FrameDD &fr, int ix, int iy) {
   const float x = ix + .5f, y = iy + .5f;
   bool out = false;
@@ -1805,7 +1805,6 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       }
       const int n = __popc(need);
       const int take = min(n, chunkLeft);
-      bool culled = false;
       const int rank = __popc(need & ((1u << lane) - 1u));
       if (((need >> lane) & 1u) && rank < take) {
         const FrameDD &fr = jobs[chunkJob].fr;
@@ -1813,7 +1812,14 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
         chunkPixel(fr, chunkBase + rank, ix, iy);
         if (pixelMisses(fr, ix, iy)) {  // stays without a pixel
           missPixel(fr, ix, iy);
-          culled = true;
+          // counted in the lane: one atomic per chunk on one address cost a frame
+          // beside its volume more than tracing its rays (640x480, 1 spp: 43 us traced,
+          // 58 with that atomic)
+          if ((unsigned)fr.spp < 1u << 24) nRays += (unsigned)fr.spp;
+          if ((unsigned)fr.spp >= 1u << 24 || nRays >= 0x80000000u) {
+            atomicAdd(&ctr->rays, (unsigned long long)nRays + ((unsigned)fr.spp < 1u << 24 ? 0u : (unsigned)fr.spp));
+            nRays = 0;
+          }
         } else {
           const int64_t pix = (int64_t)iy * fr.width + ix;
           k = 0;
@@ -1824,8 +1830,6 @@ DEV void renderLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
         }
       }
       need = __ballot_sync(FULL, phase == LP_IDLE);
-      const int nCulled = __popc(__ballot_sync(FULL, culled));
-      if (nCulled && lane == 0) atomicAdd(&ctr->rays, (unsigned long long)nCulled * (unsigned)jobs[chunkJob].fr.spp);
       chunkBase += take;
       chunkLeft -= take;
     }

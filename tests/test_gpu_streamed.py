@@ -71,6 +71,26 @@ def test_culled_pixels_over_cameras(seed):
     check(d, 2, f"camera {seed}")
 
 
+# cameras close to the volume, in it, on the planes of its faces and turned away from
+# it: corners beside and behind the camera; cut planes through, before and beyond it
+@pytest.mark.parametrize("seed", range(60))
+def test_culled_pixels_beside_the_volume(seed):
+    rng = np.random.default_rng(1000 + seed)
+    pos = rng.uniform(-0.7, 1.7, size=3)
+    if seed % 4 == 1:
+        pos[seed % 3] = float(seed % 8 > 4)
+    if seed % 4 == 2:
+        pos[seed % 3] = (-1e-3, 1.001, -0.02, 1.3)[seed // 4 % 4]
+    target = pos + rng.normal(size=3) if seed % 3 else np.array((0.5, 0.5, 0.5)) + 2 * (pos - 0.5)
+    cam = synth.look_at(pos, target=target, fovy=float(rng.uniform(20.0, 170.0)), up=tuple(rng.normal(size=3)))
+    d = synth.scene(synth.blobs(17, seed), "f32", 61, 37, synth.tf_linear_ramp(64), 20.0, cam, ambient=1.0,
+                    bg_color=(0.1, 0.0, 0.2, 1.0))
+    if seed % 5 == 3:
+        n = rng.normal(size=3)
+        d["cut_plane"] = (*(float(x) for x in n), float(rng.choice([-6.0, -0.5, 0.2, 6.0])))
+    check(d, 2, f"camera {seed}")
+
+
 # thin to dense media: nearly every draw leaves its macrocell, or none does
 @pytest.mark.parametrize("density", [1e-3, 0.5, 8.0, 400.0, -3.0])
 @pytest.mark.parametrize("exact_log", [False, True])
