@@ -550,6 +550,7 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
     if (!ctx->graphExec || key != ctx->graphKey) {
       if (ctx->graphExec) { cudaGraphExecDestroy(ctx->graphExec); ctx->graphExec = nullptr; }
       cudaGraph_t g = nullptr;
+      std::lock_guard<std::mutex> capturing(ctx->own->capture);
       ck(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
       try {
         enqueue(ctx->stream, false);
@@ -1142,7 +1143,8 @@ BN_API void bnxGetStats(BNContext context, BNXStats *stats) {
 BN_API void bnxSetStream(BNContext context, void *s) {
   BN_TRY
   Context *c = getContext(context);
-  c->stream = s ? (cudaStream_t)s : c->ownStream;
+  c->stream = s ? (cudaStream_t)s : c->own->stream;
+  if (c->stream != c->own->stream) c->own->exclusive = false;
   BN_CATCH()
 }
 
@@ -1164,7 +1166,9 @@ BN_API void bnxSetLaunchConfig(BNContext context, int bps, int tpb) {
 
 BN_API void *bnxFrameBufferDevicePointer(BNFrameBuffer fbh) {
   BN_TRY
-  return getAs<FrameBuffer>(fbh, Object::K_FB, "BNFrameBuffer")->color.ptr;
+  auto fb = getAs<FrameBuffer>(fbh, Object::K_FB, "BNFrameBuffer");
+  fb->color.handedOut = fb->color.ptr != nullptr;
+  return fb->color.ptr;
   BN_CATCH(nullptr)
 }
 
@@ -1192,7 +1196,7 @@ BN_API void bnxVolumeSample(BNVolume vh, const float *points, int n, float *scal
   v->build();  // no-op unless the TF changed
   const VolumeDD dd = v->dd();
   const size_t un = (size_t)n;
-  DeviceBuffer dP, dS, dR;
+  DeviceBuffer dP(v->ctx), dS(v->ctx), dR(v->ctx);
   dP.resize(un * sizeof(float3));
   dS.resize(un * sizeof(float));
   dR.resize(un * sizeof(float4));

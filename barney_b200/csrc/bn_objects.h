@@ -56,8 +56,8 @@ inline std::atomic<int> &allocFailCountdown() {
 // scans) otherwise pays cudaMalloc and cudaFree of every buffer, 2 of the
 // 3.7 ms that opening a 512 MB volume took.  At most kMaxHeld bytes are held
 // (the oldest go first), all of them are freed when an allocation fails and
-// when the last context is destroyed.  A block is entered only once its
-// device is idle, as cudaFree waits for it, so it can be handed to any stream.
+// when the last context is destroyed.  A block is entered only once the work that
+// uses it is done (deviceFree), so it can be handed to any stream.
 struct DeviceBlockCache {
   static constexpr size_t kMaxHeld = (size_t)4 << 30;
   struct Block {
@@ -134,17 +134,43 @@ inline cudaError_t deviceMalloc(void **p, size_t n) {
   deviceBlockCache().flush();
   return cudaMalloc(p, size);
 }
-// n: the size deviceMalloc was asked for.
-inline void deviceFree(void *p, size_t n) {
+// A context's own stream, kept until the last of the context's buffers is gone.
+// exclusive: the context has launched on no other stream (bnxSetStream).
+// capture: held while the library captures the stream.
+struct ContextStream {
+  int device;
+  cudaStream_t stream = nullptr;
+  std::atomic<bool> exclusive{true};
+  std::mutex capture;
+  explicit ContextStream(int dev) : device(dev) {}
+  ~ContextStream() {
+    if (stream && cudaStreamDestroy(stream) != cudaSuccess) cudaGetLastError();
+  }
+  ContextStream(const ContextStream &) = delete;
+  ContextStream &operator=(const ContextStream &) = delete;
+  // Waits for the stream; false if it cannot be waited for (it is being captured).
+  bool wait() {
+    std::lock_guard<std::mutex> l(capture);
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
+        cudaStreamSynchronize(stream) == cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  }
+};
+using ContextStreamSP = std::shared_ptr<ContextStream>;
+// n: the size deviceMalloc was asked for.  on: the only stream whose work uses the
+// block; null if there may be others (an application's stream, or its own kernels on
+// a pointer it was given): the block then goes back to CUDA, which waits for them.
+// Only that stream is waited for: synchronising the device, as an earlier form did,
+// is forbidden while any stream on it is captured, and breaks that capture.
+inline void deviceFree(void *p, size_t n, ContextStream *on) {
   if (!p) return;
-  int dev = 0;
-  cudaPointerAttributes at{};
-  if (cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.device == dev &&
-      DeviceBlockCache::sizeClass(n) <= DeviceBlockCache::kMaxHeld && cudaDeviceSynchronize() == cudaSuccess) {
-    deviceBlockCache().put(p, DeviceBlockCache::sizeClass(n), dev);
+  if (on && on->exclusive && DeviceBlockCache::sizeClass(n) <= DeviceBlockCache::kMaxHeld && on->wait()) {
+    deviceBlockCache().put(p, DeviceBlockCache::sizeClass(n), on->device);
     return;
   }
-  cudaGetLastError();
   if (cudaFree(p) != cudaSuccess) cudaGetLastError();
 }
 
@@ -167,17 +193,24 @@ inline float3 F3(v3 v) { return make_float3(v.x, v.y, v.z); }
 // ---------------------------------------------------------------------------
 // device buffer
 // ---------------------------------------------------------------------------
+struct Context;
+ContextStreamSP contextStream(Context *c);
+
 struct DeviceBuffer {
   void *ptr = nullptr;
   size_t bytes = 0;
-  DeviceBuffer() = default;
+  bool handedOut = false;  // the application has the pointer
+  ContextStreamSP on;
+  explicit DeviceBuffer(ContextStreamSP s) : on(std::move(s)) {}
+  explicit DeviceBuffer(Context *c) : on(contextStream(c)) {}
   DeviceBuffer(const DeviceBuffer &) = delete;
   DeviceBuffer &operator=(const DeviceBuffer &) = delete;
   ~DeviceBuffer() { release(); }
   void release() {
-    deviceFree(ptr, bytes);
+    deviceFree(ptr, bytes, handedOut ? nullptr : on.get());
     ptr = nullptr;
     bytes = 0;
+    handedOut = false;
   }
   void resize(size_t n) {
     if (n == bytes && ptr) return;
@@ -186,8 +219,6 @@ struct DeviceBuffer {
     bytes = n;
   }
 };
-
-struct Context;
 
 // NVTX range for the length of a scope: the host stages of a frame (render,
 // batch, server slice, macrocell build, read-back) show up as named ranges
@@ -229,7 +260,7 @@ struct Data : Object {
 struct TextureData : Object {
   int type = VOX_F32;
   int dims[3] = {0, 0, 0};
-  DeviceBuffer buf;
+  DeviceBuffer buf{ctx};
   explicit TextureData(Context *c) : Object(c, K_TEXDATA) {}
 };
 
@@ -285,7 +316,7 @@ struct Volume : Object {
   bool needsMajorantRebuild = false;
   bool built = false;
   int mcDims[3] = {0, 0, 0};
-  DeviceBuffer tfBuf, ranges, majorants, occupied;
+  DeviceBuffer tfBuf{ctx}, ranges{ctx}, majorants{ctx}, occupied{ctx};
   explicit Volume(Context *c) : Object(c, K_VOLUME) {}
   bool set1i(const std::string &m, int v) override {  // Volume.cpp:36-50
     if (m == "bnx.majorantRoundUp") { majorantRoundUp = v ? 1 : 0; needsMajorantRebuild = true; return true; }
@@ -355,7 +386,7 @@ struct IsoSurface : Object {
   std::shared_ptr<Material> material;
   // macrocell scalar ranges of the field, built when no volume of the group
   // provides them (StructuredData::buildMCs, StructuredData.cu:71-96)
-  DeviceBuffer ranges;
+  DeviceBuffer ranges{ctx};
   int mcDims[3] = {0, 0, 0};
   const StructuredField *rangesOf = nullptr;  // the field, texture and dims the ranges were built for
   const TextureData *rangesTex = nullptr;
@@ -502,7 +533,7 @@ struct FrameBuffer : Object {
   int colorFormat = FMT_RGBA8;
   uint32_t accumID = 0;
   uint64_t anariFrameEpoch = ~0ull;  // the context's commitEpoch at this buffer's last bnxAnariRenderFrame
-  DeviceBuffer accum, color, comp;
+  DeviceBuffer accum{ctx}, color{ctx}, comp{ctx};
   explicit FrameBuffer(Context *c) : Object(c, K_FB) {}
 };
 
@@ -511,7 +542,7 @@ struct FrameBuffer : Object {
 // ---------------------------------------------------------------------------
 struct Context {
   int device = 0;
-  cudaStream_t ownStream = nullptr;
+  ContextStreamSP own;
   cudaStream_t stream = nullptr;
   LaunchCounters *dCounters = nullptr;
   StreamRing ring;  // of this context's plain render launches (kept: 16 KB per resident warp)
@@ -521,7 +552,7 @@ struct Context {
   BNXStats stats{};
   // batch path: job table + chunk prefix (device, and pinned host mirrors a
   // captured graph copies from), and the cached graph of the last batch shape
-  DeviceBuffer batchJobs, batchChunks;
+  DeviceBuffer batchJobs{own}, batchChunks{own};
   JobDD *hostJobs = nullptr;
   int *hostChunks = nullptr;
   LaunchCounters *hostCounters = nullptr;
@@ -536,10 +567,10 @@ struct Context {
   std::mutex mutex;
   std::unordered_map<Object *, std::pair<ObjectSP, int>> handles;  // app references
 
-  explicit Context(int dev) : device(dev) {
+  explicit Context(int dev) : device(dev), own(std::make_shared<ContextStream>(dev)) {
     ck(cudaSetDevice(dev), "cudaSetDevice");
-    ck(cudaStreamCreateWithFlags(&ownStream, cudaStreamNonBlocking), "cudaStreamCreate");
-    stream = ownStream;
+    ck(cudaStreamCreateWithFlags(&own->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    stream = own->stream;
     ck(deviceMalloc((void **)&dCounters, sizeof(LaunchCounters)), "cudaMalloc counters");
     ck(cudaMemset(dCounters, 0, sizeof(LaunchCounters)), "cudaMemset");
     int sms = 0;
@@ -558,9 +589,8 @@ struct Context {
     if (hostCounters) cudaFreeHost(hostCounters);
     handles.clear();
     for (auto &e : ev) if (e) cudaEventDestroy(e);
-    deviceFree(dCounters, sizeof(LaunchCounters));
-    deviceFree(ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4));
-    if (ownStream) cudaStreamDestroy(ownStream);
+    deviceFree(dCounters, sizeof(LaunchCounters), own.get());
+    deviceFree(ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4), own.get());
     cudaGetLastError();  // nothing of a destroyed context may leak into later calls
   }
   void activate() { ck(cudaSetDevice(device), "cudaSetDevice"); }
@@ -570,6 +600,8 @@ struct Context {
     return (BNObject)o.get();
   }
 };
+
+inline ContextStreamSP contextStream(Context *c) { return c ? c->own : nullptr; }
 
 extern std::mutex g_ctxMutex;
 extern std::unordered_map<Context *, std::unique_ptr<Context>> g_contexts;

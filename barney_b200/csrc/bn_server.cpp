@@ -66,8 +66,10 @@ struct BufferPool {
   std::multimap<size_t, void *> freeDevice;
   std::vector<Chunk> chunks;
   size_t deviceBytesHeld = 0;
+  ContextStreamSP on;
+  explicit BufferPool(ContextStreamSP s) : on(std::move(s)) {}
   ~BufferPool() {
-    for (auto &c : chunks) deviceFree(c.base, c.size);
+    for (auto &c : chunks) deviceFree(c.base, c.size, on.get());
   }
   void *getDevice(size_t n) {
     const size_t need = (n + 255) & ~(size_t)255;
@@ -123,7 +125,7 @@ struct Server {
   long long nextId = 0;
   size_t bytesInUse = 0, peakBytes = 0;
   bool stop = false;
-  BufferPool pool;
+  BufferPool pool{ctx->own};
   std::thread worker;
   // statistics
   std::vector<double> latenciesMs, queueWaitsMs;
@@ -157,7 +159,10 @@ struct Server {
     if (worker.joinable()) worker.join();
     for (auto &r : active) releaseDevice(*r);
     for (auto &kv : finished) releaseResult(*kv.second);
-    if (copyStream) cudaStreamDestroy(copyStream);
+    if (copyStream) {  // the pool's chunks wait for the context's stream only
+      cudaStreamSynchronize(copyStream);
+      cudaStreamDestroy(copyStream);
+    }
     if (trace) std::fclose(trace);
     cudaGetLastError();
   }

@@ -1,16 +1,17 @@
 """Freed device blocks are kept for the next allocation of their size: volumes
 opened one after another in reused memory render as in fresh memory, an
-injected allocation failure is not hidden by a kept block, and the last
-context's end gives the memory back."""
+injected allocation failure is not hidden by a kept block, the last context's
+end gives the memory back, and a release disturbs no stream capture."""
 import os
 import subprocess
 import sys
+import threading
 
 import numpy as np
 import pytest
 
 from barney_b200 import synth
-from tests.helpers import assert_bitexact, oracle_render
+from tests.helpers import assert_bitexact, oracle_render, small_noise_scene
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +61,110 @@ assert free() >= before, "nothing is held without a context"
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr
+
+
+def test_release_during_an_applications_capture():
+    import torch
+    import barney_b200 as bn
+    ctx = bn.Context()
+    d = small_noise_scene(n=16, w=24, h=16)
+    r = bn.VolumeRenderer(d, context=ctx)
+    r.render()
+    x = torch.zeros(64, device="cuda")
+    s, g, errors = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+
+    def work():
+        try:
+            r.resize(40, 30)
+            r.close()
+            r2 = bn.VolumeRenderer(d, context=ctx)
+            r2.render()
+            r2.close()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode="thread_local")
+        x.add_(1)
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        x.add_(1)
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    ctx.close()
+    assert not errors
+    assert (x == 2).all()
+
+
+def test_release_while_another_context_captures():
+    import barney_b200 as bn
+    scenes = [small_noise_scene(n=16, w=24, h=16 + i) for i in range(6)]
+    a, b = bn.Context(), bn.Context()
+    rs = [bn.VolumeRenderer(d, context=a) for d in scenes]
+    for r in rs:
+        r.set_spp(2)
+    stop, errors = threading.Event(), []
+
+    def opens():
+        try:
+            while not stop.is_set():
+                bn.VolumeRenderer(scenes[0], context=b).close()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    t = threading.Thread(target=opens)
+    t.start()
+    try:
+        for i in range(200):  # another batch shape every time: a capture each
+            n = 1 + i % 6
+            for r in rs[:n]:
+                r.accum_reset()
+            a.render_batch(rs[:n])
+    finally:
+        stop.set()
+        t.join()
+    assert not errors
+    for r, d in zip(rs, scenes):
+        assert_bitexact(r.read(), oracle_render(d, 2)[0], "batch beside releases")
+        r.close()
+    b.close()
+    a.close()
+
+
+def test_blocks_an_application_may_still_use_go_back_to_cuda():
+    """A colour pointer handed out, and work on an application's stream: the
+    release waits for them and the next allocation does not reuse the block."""
+    import torch
+    import barney_b200 as bn
+    d = small_noise_scene(n=16, w=256, h=256)
+    ctx = bn.Context()
+    r = bn.VolumeRenderer(d, context=ctx)
+    r.render()
+    ref = r.read()
+    ptr = ctx.L.bnxFrameBufferDevicePointer(r.fb)
+    dst = torch.zeros((256, 256, 4), device="cuda")
+    libcudart = _cudart()
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(100_000_000)  # some 50 ms before the application's copy
+        assert libcudart.cudaMemcpyAsync(dst.data_ptr(), ptr, dst.numel() * 4, 3, s.cuda_stream) == 0
+    r.close()
+    r = bn.VolumeRenderer(dict(d, bg_color=(1.0, 0.5, 0.25, 1.0)), context=ctx)
+    r.render()
+    torch.cuda.synchronize()
+    assert_bitexact(dst.cpu().numpy(), ref, "the application's copy")
+    r.close()
+    ctx.close()
+
+
+def _cudart():
+    import ctypes
+    import torch  # noqa: F401
+    path = next(l.split()[-1] for l in open("/proc/self/maps") if "libcudart.so" in l)
+    lib = ctypes.CDLL(path)
+    lib.cudaMemcpyAsync.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p]
+    return lib
