@@ -50,7 +50,7 @@ EXPORTS = [
     "bnBuild", "bnCameraCreate", "bnRendererCreate", "bnFrameBufferCreate", "bnFrameBufferResize",
     "bnFrameBufferRead", "bnFrameBufferGetSize", "bnAccumReset", "bnRender", "bnGetLastError",
     "bnGetLastErrorString", "bnClearLastError", "bnxGetStats", "bnxSetStream", "bnxGetStream",
-    "bnxSetLaunchConfig", "bnxFrameBufferDevicePointer", "bnxVolumeGetMacrocells", "bnxVolumeSample", "bnxSetRegrouping",
+    "bnxSetLaunchConfig", "bnxSetMemoryCache", "bnxFrameBufferDevicePointer", "bnxVolumeGetMacrocells", "bnxVolumeSample", "bnxSetRegrouping",
     "bnxRenderStructuredNoAlloc", "bnxSetScheduling", "bnxBoundsViolations", "bnxInjectAllocationFailure", "bnxFrameBufferCheckpointSize",
     "bnxFrameBufferCheckpoint", "bnxFrameBufferRestore", "bnxRenderBatch", "bnxSetBatchGraphs", "bnxAutotuneBatch",
     "bnxServerCreate", "bnxServerDestroy", "bnxServerSubmit", "bnxServerWait", "bnxServerGetStats",
@@ -203,7 +203,7 @@ def lib(build_if_missing=True):
         "bnAccumReset": ([P], None), "bnRender": ([P, P, P, P], None), "bnGetLastError": ([], I),
         "bnGetLastErrorString": ([], S), "bnClearLastError": ([], None),
         "bnxGetStats": ([P, P], None), "bnxSetStream": ([P, P], None), "bnxGetStream": ([P], P),
-        "bnxSetLaunchConfig": ([P, I, I], None), "bnxFrameBufferDevicePointer": ([P], P),
+        "bnxSetLaunchConfig": ([P, I, I], None), "bnxSetMemoryCache": ([P, ctypes.c_size_t], None), "bnxFrameBufferDevicePointer": ([P], P),
         "bnxVolumeGetMacrocells": ([P, P, P, P], None), "bnxVolumeSample": ([P, P, I, P, P, I], None),
         "bnxRenderStructuredNoAlloc": ([P, P], I),
         "bnxSetScheduling": ([P, I], None), "bnxSetRegrouping": ([P, I], None), "bnxBoundsViolations": ([P], ctypes.c_longlong),
@@ -287,6 +287,11 @@ class Context:
 
     def set_graphs(self, enable):
         self.L.bnxSetBatchGraphs(self.ctx, int(enable))
+        check()
+
+    def set_memory_cache(self, max_bytes):
+        """Released device memory kept for reuse (bnxSetMemoryCache; 0: none)."""
+        self.L.bnxSetMemoryCache(self.ctx, int(max_bytes))
         check()
 
     def stats(self):

@@ -406,7 +406,7 @@ static void render(Context *ctx, Renderer &r, Model &m, Camera &cam, FrameBuffer
   if (job.fr.spp <= 0) return;
   ck(cudaMemsetAsync(ctx->dCounters, 0, sizeof(LaunchCounters), ctx->stream), "counter reset");
   ck(cudaEventRecord(ctx->ev[0], ctx->stream), "event");
-  ck(launchRenderJob(ctx, job, ctx->stream), "render kernel");
+  ck(withoutCacheIfFull([&] { return launchRenderJob(ctx, job, ctx->stream); }), "render kernel");
   ck(cudaEventRecord(ctx->ev[1], ctx->stream), "event");
   fb.accumID += job.fr.spp;
   ck(launchResolve((const float4 *)fb.accum.ptr, fb.width * fb.height, (int)fb.accumID, fb.colorFormat, fb.color.ptr,
@@ -560,7 +560,7 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
         throw;
       }
       ck(cudaStreamEndCapture(ctx->stream, &g), "graph capture");
-      cudaError_t e = cudaGraphInstantiate(&ctx->graphExec, g, 0);
+      cudaError_t e = withoutCacheIfFull([&] { return cudaGraphInstantiate(&ctx->graphExec, g, 0); });
       cudaGraphDestroy(g);
       ck(e, "graph instantiate");
       ctx->graphKey = key;
@@ -624,13 +624,6 @@ BN_API void bnContextDestroy(BNContext context) {
     owned = std::move(g_contexts[c]);
     g_contexts.erase(c);
   }
-  owned.reset();
-  bool last;
-  {
-    std::lock_guard<std::mutex> l(g_ctxMutex);
-    last = g_contexts.empty();
-  }
-  if (last) deviceBlockCache().flush();
   BN_CATCH()
 }
 
@@ -1152,6 +1145,14 @@ BN_API void *bnxGetStream(BNContext context) {
   BN_TRY
   return (void *)getContext(context)->stream;
   BN_CATCH(nullptr)
+}
+
+BN_API void bnxSetMemoryCache(BNContext context, size_t maxBytes) {
+  BN_TRY
+  Context *c = getContext(context);
+  c->own->cacheLimit = std::min(maxBytes, DeviceBlockCache::kMaxHeld);
+  deviceBlockCache().trim(c->own->cacheLimit);
+  BN_CATCH()
 }
 
 BN_API void bnxSetLaunchConfig(BNContext context, int bps, int tpb) {

@@ -54,10 +54,12 @@ inline std::atomic<int> &allocFailCountdown() {
 // Freed device blocks kept for the next allocation of their size class: a
 // client that opens volume after volume of one size (time steps, a browser of
 // scans) otherwise pays cudaMalloc and cudaFree of every buffer, 2 of the
-// 3.7 ms that opening a 512 MB volume took.  At most kMaxHeld bytes are held
-// (the oldest go first), all of them are freed when an allocation fails and
-// when the last context is destroyed.  A block is entered only once the work that
-// uses it is done (deviceFree), so it can be handed to any stream.
+// 3.7 ms that opening a 512 MB volume took.  At most kMaxHeld bytes are held, or
+// what the releasing context allows (bnxSetMemoryCache); the oldest go first.  All
+// go when the last context ends and when an allocation of this library fails;
+// other users of the device get them by bnxSetMemoryCache only.  A block is entered
+// only once the work that uses it is done (deviceFree), so it can be handed to any
+// stream.
 struct DeviceBlockCache {
   static constexpr size_t kMaxHeld = (size_t)4 << 30;
   struct Block {
@@ -68,6 +70,7 @@ struct DeviceBlockCache {
   std::mutex m;
   std::deque<Block> blocks;
   size_t held = 0;
+  int users = 0;  // contexts; without one nothing is held
   // cudaMalloc's own granularity: 2 MiB, 512 B below 1 MiB
   static size_t sizeClass(size_t n) {
     const size_t g = n < ((size_t)1 << 20) ? 512 : (size_t)2 << 20;
@@ -84,35 +87,76 @@ struct DeviceBlockCache {
       }
     return nullptr;
   }
-  void put(void *p, size_t n, int device) {
-    std::vector<void *> drop;
+  // False if the block is not taken; older ones go until at most `limit` bytes are held.
+  bool put(void *p, size_t n, int device, size_t limit) {
+    if (n > limit) return false;
+    std::vector<Block> drop;
     {
       std::lock_guard<std::mutex> l(m);
+      if (!users) return false;
       blocks.push_back({p, n, device});
       held += n;
-      while (held > kMaxHeld) {
-        drop.push_back(blocks.front().ptr);
-        held -= blocks.front().bytes;
-        blocks.pop_front();
-      }
+      shrink(limit, drop);
     }
-    for (void *d : drop)
-      if (cudaFree(d) != cudaSuccess) cudaGetLastError();
+    give(drop);
+    return true;
   }
-  void flush() {
-    std::deque<Block> all;
+  // Gives back the oldest blocks until at most `limit` bytes are held; true if there were any.
+  bool trim(size_t limit) {
+    std::vector<Block> drop;
     {
       std::lock_guard<std::mutex> l(m);
-      all.swap(blocks);
-      held = 0;
+      shrink(limit, drop);
     }
-    for (auto &b : all)
+    give(drop);
+    return !drop.empty();
+  }
+  void enter() {
+    std::lock_guard<std::mutex> l(m);
+    users++;
+  }
+  void leave() {
+    std::vector<Block> drop;
+    {
+      std::lock_guard<std::mutex> l(m);
+      if (--users == 0) shrink(0, drop);
+    }
+    give(drop);
+  }
+
+ private:
+  void shrink(size_t limit, std::vector<Block> &drop) {
+    while (held > limit) {
+      drop.push_back(blocks.front());
+      held -= blocks.front().bytes;
+      blocks.pop_front();
+    }
+  }
+  static void give(const std::vector<Block> &drop) {
+    for (auto &b : drop)
       if (cudaFree(b.ptr) != cudaSuccess) cudaGetLastError();
   }
 };
 inline DeviceBlockCache &deviceBlockCache() {
   static DeviceBlockCache *c = new DeviceBlockCache;  // never destroyed: buffers may be freed at exit
   return *c;
+}
+struct DeviceBlockCacheUser {
+  DeviceBlockCacheUser() { deviceBlockCache().enter(); }
+  ~DeviceBlockCacheUser() { deviceBlockCache().leave(); }
+  DeviceBlockCacheUser(const DeviceBlockCacheUser &) = delete;
+  DeviceBlockCacheUser &operator=(const DeviceBlockCacheUser &) = delete;
+};
+// A call that may need device memory of its own, again without the held blocks if
+// it found none.
+template <typename F>
+inline cudaError_t withoutCacheIfFull(F call) {
+  cudaError_t e = call();
+  if (e == cudaErrorMemoryAllocation && deviceBlockCache().trim(0)) {
+    cudaGetLastError();
+    e = call();
+  }
+  return e;
 }
 // Device memory of the current device, or the injected failure; freed with deviceFree.
 inline cudaError_t deviceMalloc(void **p, size_t n) {
@@ -128,19 +172,17 @@ inline cudaError_t deviceMalloc(void **p, size_t n) {
   if (e != cudaSuccess) return e;
   const size_t size = DeviceBlockCache::sizeClass(n);
   if ((*p = deviceBlockCache().take(size, dev))) return cudaSuccess;
-  e = cudaMalloc(p, size);
-  if (e != cudaErrorMemoryAllocation) return e;
-  cudaGetLastError();
-  deviceBlockCache().flush();
-  return cudaMalloc(p, size);
+  return withoutCacheIfFull([&] { return cudaMalloc(p, size); });
 }
 // A context's own stream, kept until the last of the context's buffers is gone.
 // exclusive: the context has launched on no other stream (bnxSetStream).
+// cacheLimit: bytes the block cache may hold after a release of this context.
 // capture: held while the library captures the stream.
 struct ContextStream {
   int device;
   cudaStream_t stream = nullptr;
   std::atomic<bool> exclusive{true};
+  std::atomic<size_t> cacheLimit{DeviceBlockCache::kMaxHeld};
   std::mutex capture;
   explicit ContextStream(int dev) : device(dev) {}
   ~ContextStream() {
@@ -167,10 +209,10 @@ using ContextStreamSP = std::shared_ptr<ContextStream>;
 // is forbidden while any stream on it is captured, and breaks that capture.
 inline void deviceFree(void *p, size_t n, ContextStream *on) {
   if (!p) return;
-  if (on && on->exclusive && DeviceBlockCache::sizeClass(n) <= DeviceBlockCache::kMaxHeld && on->wait()) {
-    deviceBlockCache().put(p, DeviceBlockCache::sizeClass(n), on->device);
+  const size_t size = DeviceBlockCache::sizeClass(n);
+  if (on && on->exclusive && size <= on->cacheLimit && on->wait() &&
+      deviceBlockCache().put(p, size, on->device, on->cacheLimit))
     return;
-  }
   if (cudaFree(p) != cudaSuccess) cudaGetLastError();
 }
 
@@ -541,6 +583,7 @@ struct FrameBuffer : Object {
 // context
 // ---------------------------------------------------------------------------
 struct Context {
+  DeviceBlockCacheUser cacheUser;  // leaves when every buffer of the context is released
   int device = 0;
   ContextStreamSP own;
   cudaStream_t stream = nullptr;

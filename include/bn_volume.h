@@ -278,6 +278,17 @@ BN_API void bnxGetStats(BNContext context, BNXStats *stats);
    selects the context's own stream. */
 BN_API void bnxSetStream(BNContext context, void *cudaStream);
 BN_API void *bnxGetStream(BNContext context);
+/* Device memory that released objects of a context held (textures, macrocell
+   grids, frame buffers, server buffers) is kept for the next allocation of its
+   size, by any context on the device: at most 4 GiB for the whole process, given
+   back to CUDA when the last context is destroyed and when an allocation of this
+   library fails.  Other users of the device (the application's own cudaMalloc,
+   other processes) do not get it before.  This call gives back what is held
+   beyond maxBytes, and lets later releases of this context keep no more than that
+   (at most the 4 GiB; 0: they go back to CUDA at once).  Contexts given a stream by
+   bnxSetStream, and colour buffers whose pointer was handed out, always release
+   to CUDA. */
+BN_API void bnxSetMemoryCache(BNContext context, size_t maxBytes);
 /* Deadline of bnRender and bnxRenderBatch (0: none), counted from the call.
    When a frame is still running at the deadline, the render kernel is told
    to stop (every warp quits at its next pixel chunk), the frame buffer's

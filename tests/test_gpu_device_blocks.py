@@ -63,6 +63,35 @@ assert free() >= before, "nothing is held without a context"
     assert p.returncode == 0, p.stderr
 
 
+def test_memory_goes_back_on_request_and_after_the_last_context():
+    code = """
+import torch, barney_b200 as bn
+free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info()[0])[1]
+vox = torch.zeros((256, 512, 512), device="cuda"); torch.cuda.synchronize()
+MB = 1 << 20
+ctx = bn.Context()
+def cycle():
+    t = ctx.L.bnTextureData3DCreate(ctx.ctx, 0, bn.BN_FLOAT32, 512, 512, 256, vox.data_ptr()); bn.check()
+    ctx.L.bnRelease(t); bn.check()
+cycle(); ctx.set_memory_cache(0); before = free()
+cycle()
+assert before - free() <= 8 * MB, "with no cache a release is given back at once"
+ctx.set_memory_cache(300 * MB)
+cycle()
+assert before - free() >= 256 * MB, "kept"
+other = bn.Context(); other.set_memory_cache(0); other.close()
+assert before - free() <= 8 * MB, "trimmed"
+cycle(); cycle()
+s = bn.Server(ctx, max_slots=2, slice_waves=1); s.reserve(512 * MB)
+ctx.close()
+s.close()
+assert free() >= before - 8 * MB, "the server's buffers, released after the last context"
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+
+
 def test_release_during_an_applications_capture():
     import torch
     import barney_b200 as bn
