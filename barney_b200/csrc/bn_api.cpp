@@ -386,13 +386,14 @@ static bool waitWithDeadline(Context *ctx, cudaEvent_t done, std::chrono::steady
 static bool plainJob(const JobDD &job) {
   return !job.v.iso.enabled && job.fr.maxVolumeBounces <= 0 && !job.v.pv.enabled;
 }
-// Plain jobs run the regrouped kernel unless the context turned it off
-// (bnxSetRegrouping); the per-lane kernel is the same frame.
+// Plain jobs run the streamed kernel, or the regrouped one if the context asks for
+// it (bnxSetRegrouping); both give the same frame.
 static cudaError_t launchRenderJob(Context *ctx, const JobDD &job, cudaStream_t s) {
   const bool plain = plainJob(job);
   if (plain && ctx->sched.regrouped)
     return job.fr.fastMath ? fastmath::launchRenderRegrouped(job.v, job.fr, ctx->dCounters, s)
                            : launchRenderRegrouped(job.v, job.fr, ctx->dCounters, s);
+  if (plain) ctx->ensureRing();
   if (job.fr.fastMath && plain)
     return fastmath::launchRender(job.v, job.fr, ctx->dCounters, ctx->blocksPerSM, ctx->threadsPerBlock, s, ctx->sched,
                                   ctx->ring);
@@ -509,6 +510,7 @@ void renderBatch(Context *ctx, const std::vector<BatchEntry> &entries) {
   // the TF in shared memory, and a plain resolve -- the same frame as the
   // batch kernel's, faster
   const bool solo = n == 1 && !ctx->useGraphs;
+  if (extended == 0 && !solo) ctx->ensureRing();  // not under capture
   auto enqueue = [&](cudaStream_t s, bool timed) {
     if (solo) {
       const JobDD &job = ctx->hostJobs[0];

@@ -587,8 +587,9 @@ struct Context {
   int device = 0;
   ContextStreamSP own;
   cudaStream_t stream = nullptr;
+  DeviceBuffer counters{own}, rings{own};
   LaunchCounters *dCounters = nullptr;
-  StreamRing ring;  // of this context's plain render launches (kept: 16 KB per resident warp)
+  StreamRing ring;  // of this context's plain render launches: from the first one on, 16 KB per resident warp
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   int blocksPerSM = 0, threadsPerBlock = 128;
   SchedDD sched;
@@ -614,13 +615,33 @@ struct Context {
     ck(cudaSetDevice(dev), "cudaSetDevice");
     ck(cudaStreamCreateWithFlags(&own->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     stream = own->stream;
-    ck(deviceMalloc((void **)&dCounters, sizeof(LaunchCounters)), "cudaMalloc counters");
+    counters.resize(sizeof(LaunchCounters));
+    dCounters = (LaunchCounters *)counters.ptr;
     ck(cudaMemset(dCounters, 0, sizeof(LaunchCounters)), "cudaMemset");
+    try {
+      for (auto &e : ev) ck(cudaEventCreate(&e), "cudaEventCreate");
+    } catch (...) {
+      for (auto &e : ev) if (e) cudaEventDestroy(e);
+      throw;
+    }
+  }
+  // Ring memory for the plain kernels.  A device that has not enough left for every
+  // resident warp (74 MiB) gets a smaller one: launches then use fewer warps.
+  void ensureRing() {
+    if (ring.ptr) return;
     int sms = 0;
-    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    ring.warps = sms * kStreamWarpsPerSM;
-    ck(deviceMalloc((void **)&ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4)), "cudaMalloc path rings");
-    for (auto &e : ev) ck(cudaEventCreate(&e), "cudaEventCreate");
+    ck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
+    for (int warps = sms * kStreamWarpsPerSM;; warps /= 2) {
+      try {
+        rings.resize((size_t)warps * kStreamRing * sizeof(float4));
+      } catch (const Error &e) {
+        if (e.code != E_OOM || warps / 2 < kRenderMaxThreads / 32) throw;
+        continue;
+      }
+      ring.ptr = (float4 *)rings.ptr;
+      ring.warps = warps;
+      return;
+    }
   }
   ~Context() {
     cudaSetDevice(device);
@@ -632,8 +653,6 @@ struct Context {
     if (hostCounters) cudaFreeHost(hostCounters);
     handles.clear();
     for (auto &e : ev) if (e) cudaEventDestroy(e);
-    deviceFree(dCounters, sizeof(LaunchCounters), own.get());
-    deviceFree(ring.ptr, (size_t)ring.warps * kStreamRing * sizeof(float4), own.get());
     cudaGetLastError();  // nothing of a destroyed context may leak into later calls
   }
   void activate() { ck(cudaSetDevice(device), "cudaSetDevice"); }

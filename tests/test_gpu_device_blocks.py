@@ -92,6 +92,65 @@ assert free() >= before - 8 * MB, "the server's buffers, released after the last
     assert p.returncode == 0, p.stderr
 
 
+def test_path_rings_come_with_the_first_plain_frame():
+    code = """
+import torch, barney_b200 as bn
+from barney_b200 import synth
+free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info()[0])[1]
+MB = 1 << 20
+d = synth.config2(vol=synth.value_noise(16, 0), width=24, height=16)
+keep = bn.Context()
+for bounces in (0, 2):  # the kernels' code is loaded on their first launch
+    r = bn.VolumeRenderer(dict(d, max_volume_bounces=bounces), context=keep); r.render(); r.close()
+before = free()
+ctxs = [bn.Context() for _ in range(4)]
+assert before - free() <= 8 * MB, "contexts alone"
+rs = [bn.VolumeRenderer(dict(d, max_volume_bounces=2), context=c) for c in ctxs]
+for r in rs: r.render()
+assert before - free() <= 32 * MB, "multi-scatter frames need no rings"
+r = bn.VolumeRenderer(d, context=ctxs[0]); r.render()
+assert 64 * MB <= before - free() <= 112 * MB, "one context's rings"
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+
+
+def test_failed_allocations_of_a_context():
+    """A context that cannot be created leaves nothing behind, and one whose
+    path rings find no memory renders the same frames with smaller ones."""
+    import barney_b200 as bn
+    L = bn.lib()
+    d = small_noise_scene(n=20, w=301, h=203)
+    try:
+        L.bnxInjectAllocationFailure(0)
+        assert not L.bnContextCreate(1, None, 0, None)
+        assert L.bnGetLastError() == 6
+        L.bnClearLastError()
+        for batch in (False, True):
+            ctx = bn.Context()
+            rs = [bn.VolumeRenderer(d, context=ctx) for _ in range(2)]
+            for r in rs:
+                r.set_spp(9)
+            if batch:
+                L.bnxInjectAllocationFailure(2)  # the batch's job and chunk tables, then the rings
+                ctx.render_batch(rs)
+            else:
+                L.bnxInjectAllocationFailure(0)
+                rs[0].render()
+            bn.check()
+            assert_bitexact(rs[0].read(), oracle_render(d, 9)[0], f"smaller rings, batch {batch}")
+            # the injected failure was the rings': none is left for this one
+            t = L.bnTextureData3DCreate(ctx.ctx, 0, bn.BN_FLOAT32, 2, 2, 2, np.zeros(8, np.float32).ctypes.data)
+            bn.check()
+            L.bnRelease(t)
+            for r in rs:
+                r.close()
+            ctx.close()
+    finally:
+        L.bnxInjectAllocationFailure(-1)
+
+
 def test_release_during_an_applications_capture():
     import torch
     import barney_b200 as bn
