@@ -351,10 +351,12 @@ DEV float2 macrocellRange(const VolumeDD &v, int64_t tid, int64_t n, const float
   const int x0 = mx * kCellsPerMC, y0 = my * kCellsPerMC, z0 = mz * kCellsPerMC;
   const int x1 = min(x0 + kCellsPerMC, v.numScalars.x - 1);
   const int y1 = min(y0 + kCellsPerMC, v.numScalars.y - 1);
-  const int z1 = valid ? min(z0 + kCellsPerMC, v.numScalars.z - 1) : z0 - 1;
   const int64_t nx = v.numScalars.x, nxy = (int64_t)v.numScalars.x * v.numScalars.y;
+  // no rows past the last macrocell, or in the bounds-checked build after a violation:
+  // the lane stays, as its warp shuffles below
+  const int zLast = min(z0 + kCellsPerMC, v.numScalars.z - 1);
+  const int z1 = valid && BNB_IN(x1 + nx * y1 + nxy * zLast, nxy * v.numScalars.z) ? zLast : z0 - 1;
   float lo = kInf, hi = -kInf;
-  if (valid && !BNB_IN(x1 + nx * y1 + nxy * z1, nxy * v.numScalars.z)) return make_float2(lo, hi);
   if (nx % 8 != 0 || (uintptr_t)v.voxels % 16 != 0) {
     for (int z = z0; z <= z1; z++)
       for (int y = y0; y <= y1; y++) {

@@ -32,6 +32,10 @@ scenes = [
 ]
 ragged = synth.value_noise(21, 3)[:, 2:15, 4:13].copy()
 scenes.append(dict(synth.config2(vol=ragged, width=15, height=11), spacing=(1 / 8, 1 / 12, 1 / 20)))
+# rows read as vectors: a warp of macrocells, one that ends inside it, and more
+for shape, dtype in (((10, 9, 264), "f32"), ((9, 17, 248), "u8"), ((3, 12, 520), "f16"), ((12, 3, 8), "u16")):
+    vol = synth.to_storage(np.random.default_rng(1).random(shape).astype(np.float32), dtype)
+    scenes.append(synth.scene(vol, dtype, 18, 13, synth.tf_linear_ramp(64), 20.0, synth.DEFAULT_CAMERA))
 ctx = bn.Context()
 assert ctx.L.bnxBoundsViolations(ctx.ctx) == 0, "bounds-checked build expected"
 for i, d in enumerate(scenes):
