@@ -2193,6 +2193,7 @@ DEV void retireSlot(const FrameDD &fr, StreamWarp &sw, int s, const float4 *ring
   int waves = sw.waves[s], accumID = fr.accumID0 + sw.wave[s];
   // the slot's entries to shared memory: one round trip to L2, not one a wave
   const int total = n * waves;
+  const bool fits = BNB_IN(total, kStreamSlotPaths + 1);
   for (int i = lane; i < total && i < kStreamSlotPaths; i += 32) ringFetch(&sw.entry[i], ring + s * kStreamSlotPaths + i);
   int ix = 0, iy = 0;
   bool mine = lane < sw.count[s];
@@ -2211,12 +2212,13 @@ DEV void retireSlot(const FrameDD &fr, StreamWarp &sw, int s, const float4 *ring
   const bool whole = !issues && bg.w == 1.f && bg.x <= 0.f && bg.y <= 0.f && bg.z <= 0.f && accumID > 0 &&
                      acc.w >= 0.f && acc.w == truncf(acc.w) && acc.w <= 8388608.f && waves <= 8388608;
   if (whole) acc.w += (float)waves;
-  if (!mine || whole) waves = 0;
+  if (!mine || whole || !fits) waves = 0;
   const float4 *entry = sw.entry + (issues ? __popc(m & ((1u << lane) - 1u)) : 0);
   ringFetchWait();
   __syncwarp();
 #pragma unroll 1
   for (; waves > 0; waves--, accumID++) {
+    if (!BNB_IN(entry - sw.entry, kStreamSlotPaths)) break;
     float4 f = *entry;
     if (issues) entry += n;
     const bool missed = !issues || f.w == kPathMissed;
@@ -2296,17 +2298,17 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       if (phase == LP_HIT && !shadow) {
         const FrameDD &fr = jobs[BATCH ? job : 0].fr;
         done = fr.emissionAbsorption;
-        if (done) {
+        if (done && BNB_IN(path, kStreamRing)) {
           const int s = path / kStreamSlotPaths;
           const float clampMax = 10.f * (1 + fr.accumID0 + sw.wave[s] + slotWave(sw, s, path % kStreamSlotPaths));
           ringStore(ring + path, make_float4(fmin_(ts.tNext.x, clampMax), fmin_(ts.tNext.y, clampMax),
                                              fmin_(ts.tNext.z, clampMax), kPathLit));
         }
-      } else if (!shadow || phase == LP_HIT) {
+      } else if ((!shadow || phase == LP_HIT) && BNB_IN(path, kStreamRing)) {
         ringStoreW(ring + path, shadow ? kPathOccluded : kPathMissed);
       }
       if (done) {
-        atomicSub(&sw.left[path / kStreamSlotPaths], 1);
+        if (BNB_IN(path, kStreamRing)) atomicSub(&sw.left[path / kStreamSlotPaths], 1);
         phase = LP_IDLE;
       }
     }
@@ -2325,11 +2327,13 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       if (phase == LP_HIT) {
         const int q = ctl.parked() + __popc(holding & below);
         const uint2 seed = sw.seed[lane];
-        sw.qA[q] = make_float4(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z, ts.t);
-        sw.qB[q] = make_float4((ts.bits & 8) ? 0.f : ts.dir.x, (ts.bits & 16) ? 0.f : ts.dir.y,
-                               (ts.bits & 32) ? 0.f : ts.dir.z, __int_as_float(path));
-        sw.qC[q] = make_float4(ts.tNext.x, ts.tNext.y, ts.tNext.z, __uint_as_float(seed.x));
-        sw.qD[q] = seed.y;
+        if (BNB_IN(q, 32)) {
+          sw.qA[q] = make_float4(ts.org.x + ts.t * ts.dir.x, ts.org.y + ts.t * ts.dir.y, ts.org.z + ts.t * ts.dir.z, ts.t);
+          sw.qB[q] = make_float4((ts.bits & 8) ? 0.f : ts.dir.x, (ts.bits & 16) ? 0.f : ts.dir.y,
+                                 (ts.bits & 32) ? 0.f : ts.dir.z, __int_as_float(path));
+          sw.qC[q] = make_float4(ts.tNext.x, ts.tNext.y, ts.tNext.z, __uint_as_float(seed.x));
+          sw.qD[q] = seed.y;
+        }
         phase = LP_IDLE;
       }
       ctl.park(__popc(holding));
@@ -2351,7 +2355,9 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
           if (mine) {
             const int i = ctl.nextPath() + rank;
             const int k = slotWave(sw, s, i);
-            const int2 p = sw.pixel[sw.pathPixel[i - k * __popc(sw.mask[s])]];
+            const int j = i - k * __popc(sw.mask[s]);
+            const int lanePixel = BNB_IN(j, __popc(sw.unitMask)) ? sw.pathPixel[j] : 0;
+            const int2 p = BNB_IN(lanePixel, sw.unitCount) ? sw.pixel[lanePixel] : make_int2(0, 0);
             pixelX = p.x;
             pixelY = p.y;
             wave = sw.wave[s] + k;
@@ -2387,7 +2393,8 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
       uint2 seed = sw.seed[lane];
       const int parked = ctl.parked();
       if (((empty >> lane) & 1u) && rank < parked) {
-        const int q = parked - 1 - rank;
+        int q = parked - 1 - rank;
+        if (!BNB_IN(q, 32)) q = 0;
         const float4 a = sw.qA[q], b = sw.qB[q], c = sw.qC[q];
         P = f3(a.x, a.y, a.z);
         tHit = a.w;
@@ -2395,11 +2402,12 @@ DEV void streamLoop(const JobDD *__restrict__ jobs, const int *__restrict__ chun
         path = __float_as_int(b.w);
         rgb = f3(c.x, c.y, c.z);
         seed = make_uint2(__float_as_uint(c.w), sw.qD[q]);
-        if (BATCH) job = sw.job[path / kStreamSlotPaths];
+        if (BATCH && BNB_IN(path, kStreamRing)) job = sw.job[path / kStreamSlotPaths];
         shade = true;
       }
       ctl.park(-min(parked, __popc(empty)));
       __syncwarp();
+      if (shade && !BNB_IN(path, kStreamRing)) shade = false, phase = LP_IDLE;
       if (shade) {
         const JobDD &J = jobs[BATCH ? job : 0];
         const int s = path / kStreamSlotPaths;

@@ -16,6 +16,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 CHILD = r"""
 import numpy as np
+import oracle
 import barney_b200 as bn
 from barney_b200 import synth
 from tests.helpers import assert_bitexact, oracle_render, small_blob_scene, small_noise_scene
@@ -46,6 +47,33 @@ for i, d in enumerate(scenes):
     ref, _, _ = oracle_render(d, 6)
     assert_bitexact(r.read(), ref, f"scene {i}")
     r.close()
+# the streamed loop's rings: several slots a unit, rings that wrap, units of 32, 16 and 8 pixels
+near = dict(camera=synth.look_at((1.1, 0.9, 1.2)))
+for d, spp in ((small_noise_scene(n=20, w=70, h=61, **near), 1), (small_noise_scene(n=20, w=70, h=61, **near), 2),
+               (small_noise_scene(n=20, w=70, h=61, **near), 65), (small_noise_scene(n=20, w=33, h=31, **near), 33),
+               (small_noise_scene(n=20, w=401, h=205, density=5.0, **near), 8), (small_blob_scene(n=20, w=1021, h=563), 8),
+               (small_blob_scene(n=20, w=61, h=43, emission_absorption=True, ambient=0.0), 19),
+               (small_noise_scene(n=20, w=61, h=43, compensated_accum=True, majorant_round_up=True), 17)):
+    r = bn.VolumeRenderer(d, color_format="float4", context=ctx)
+    r.set_spp(spp)
+    r.render()
+    acc = np.zeros((d["height"], d["width"], 4), np.float32)
+    comp = np.zeros_like(acc) if d.get("compensated_accum") else None
+    oracle.render(oracle.Scene(d), 0, spp, accum=acc, comp=comp)
+    assert_bitexact(r.read(), oracle.resolve(acc, spp, comp=comp), f"{d['width']}x{d['height']} {spp} spp")
+    r.close()
+plain = [small_noise_scene(n=[16, 20, 13][i % 3], w=40 + 23 * i, h=61 - 3 * i, dtype=["f32", "u8", "f16"][i % 3], **near)
+         for i in range(9)]
+for graphs in (False, True):
+    for n in (3, 9):  # a kernel parameter, a table
+        ctx.set_graphs(graphs)
+        rs = [bn.VolumeRenderer(d, color_format="float4", context=ctx) for d in plain[:n]]
+        for i, r in enumerate(rs):
+            r.set_spp([1, 9, 33][i % 3])
+        ctx.render_batch(rs)
+        for i, (r, d) in enumerate(zip(rs, plain)):
+            assert_bitexact(r.read(), oracle_render(d, [1, 9, 33][i % 3])[0], f"job {i}")
+            r.close()
 rs = [bn.VolumeRenderer(d, color_format="float4", context=ctx) for d in scenes[:4]]
 for r in rs:
     r.set_spp(2)
