@@ -3455,7 +3455,8 @@ static cudaError_t launchStreamT(const VolumeDD &v, const FrameDD &fr, SchedDD s
 
 #ifndef BNB_FAST_MATH
 // The lane-owned kernels: extended jobs, and plain ones on the path that has
-// no ring memory (the no-allocation entry point, without compensated sums).
+// no ring memory (the no-allocation entry point, without compensated sums or the
+// exact logarithm).
 template <int T>
 static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, SchedDD sd, LaunchCounters *ctr,
                                 int bps, int tpb, cudaStream_t s) {
@@ -3465,7 +3466,7 @@ static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, SchedDD sd
   if (sd.serviceBatch <= 0) sd.serviceBatch = lanesServiceBatch(ext);
   // kernels with and without compensated sums
   const bool cmp = fr.comp != nullptr;
-  if (ext == 0 && cmp) return cudaErrorInvalidValue;
+  if (ext == 0 && (cmp || fr.exactLog)) return cudaErrorInvalidValue;
   // isosurfaces without volume bounces or principled volumes: the smaller
   // EXT 3 kernel unless the job keeps compensated sums
   auto kern = ext == 3 && !cmp ? (fr.exactLog ? renderKernel<T, 1, 3, 0> : renderKernel<T, 0, 3, 0>)
@@ -3473,7 +3474,7 @@ static cudaError_t launchLanesT(const VolumeDD &v, const FrameDD &fr, SchedDD sd
                                 : (fr.exactLog ? renderKernel<T, 1, 2, 0> : renderKernel<T, 0, 2, 0>))
               : ext == 1 ? (cmp ? (fr.exactLog ? renderKernel<T, 1, 1, 2> : renderKernel<T, 0, 1, 2>)
                                 : (fr.exactLog ? renderKernel<T, 1, 1, 0> : renderKernel<T, 0, 1, 0>))
-                         : (fr.exactLog ? renderKernel<T, 1, 0, 0> : renderKernel<T, 0, 0, 0>);
+                         : renderKernel<T, 0, 0, 0>;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return cudaGetLastError();
