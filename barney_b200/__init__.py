@@ -562,7 +562,7 @@ class VolumeRenderer:
         check()
 
     def set_regrouping(self, enable=True):
-        """Regrouped kernel for plain jobs, or the per-lane kernel (default)."""
+        """Regrouped kernel for plain jobs, or the streamed kernel (default)."""
         self.L.bnxSetRegrouping(self.ctx, 1 if enable else 0)
         check()
 

@@ -2036,9 +2036,9 @@ __global__ void __launch_bounds__(kRenderMaxThreads, EXT >= 2 ? kRenderMinBlocks
 // host) issue no paths; they add their miss colour where they are found (three
 // quarters of the 1080p frame around a cube).
 //
-// Bound: instruction issue and fetch (65 % of issue slots, no-instruction stalls
-// 1.7 per issue).  Against the lane-owned loop on the 512^3 1080p 64-spp frame (ncu
-// on 8 spp): warp instructions 1.65 -> 0.84 G, 11.1 -> 19.3 of 32 lanes an
+// Bound: instruction issue and fetch (67 % of issue slots, no-instruction stalls
+// 1.9 per issue).  Against the lane-owned loop on the 512^3 1080p 64-spp frame (ncu
+// on 8 spp): warp instructions 1.65 -> 0.84 G, 11.1 -> 19.6 of 32 lanes an
 // instruction, kernel 14.5 -> 7.8 ms; 256^2 x 16 spp of a 64^3 volume, where a
 // pixel's waves no longer wait for one another, 1.0 -> 0.22 ms; 64 mixed jobs
 // 41 -> 24 ms.  Steps that end inside a macrocell wait for one another too: 4 -> 20
@@ -3339,9 +3339,9 @@ static int smCount() {
 
 #ifndef BNB_FAST_MATH
 // Occupancy bitmap of a majorant grid: one ballot per warp packs the
-// "majorant != 0" flags of 32 consecutive macrocells into one word.  The
-// render loop tests these bits (32 KB for a 64^3 grid, resident in L1)
-// instead of loading a majorant for every macrocell it crosses.
+// "majorant != 0" flags of 32 consecutive macrocells into one word (32 KB for a
+// 64^3 grid).  Only the regrouped kernel reads it; the other render loops load the
+// majorants themselves (walkCell).
 __global__ void __launch_bounds__(256) mcOccupancyKernel(const float *majorants, int64_t n, unsigned *occupied) {
   const int lane = threadIdx.x & 31;
   const int64_t words = (n + 31) >> 5;

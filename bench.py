@@ -64,8 +64,8 @@ def parse():
     p.add_argument("--tile-dp", action="store_true",
                    help="configs 1-3 on N GPUs: split each frame's pixel tiles across the ranks and gather "
                         "the frame over NCCL every step (strong scaling) instead of one frame per rank")
-    p.add_argument("--kernel", default="per-lane", choices=["per-lane", "regrouped"],
-                   help="render kernel of plain jobs: one pixel per lane (default) or regrouped pixel slots")
+    p.add_argument("--kernel", default="streamed", choices=["streamed", "regrouped"],
+                   help="render kernel of plain jobs: paths streamed through warps (default) or regrouped pixel slots")
     p.add_argument("--rmse", action="store_true", help="image RMSE of every storage form vs the FP64 oracle")
     p.add_argument("--rmse-size", default="96x54", help="image size of the RMSE frames")
     p.add_argument("--rmse-spp", type=int, default=4096)

@@ -278,6 +278,8 @@ BN_API void bnxGetStats(BNContext context, BNXStats *stats);
    selects the context's own stream. */
 BN_API void bnxSetStream(BNContext context, void *cudaStream);
 BN_API void *bnxGetStream(BNContext context);
+/* A context's first plain frame takes 74 MiB of device memory for the streamed
+   kernel's path rings (less where that does not fit), kept until the context ends. */
 /* Device memory that released objects of a context held (textures, macrocell
    grids, frame buffers, server buffers) is kept for the next allocation of its
    size, by any context on the device: at most 4 GiB for the whole process, given
@@ -314,16 +316,17 @@ BN_API void bnxSetLaunchConfig(BNContext context, int blocksPerSM, int threadsPe
    which wait in ring queues there (new pixels, rays to trace, collisions to
    shade, rays that ended); each warp takes up to 32 slots from one queue at
    a time, with no block-wide barrier, so that every step runs with full
-   warps.  The default (0) is the per-lane kernel (one pixel per lane;
-   bnxSetLaunchConfig and bnxSetScheduling apply to it), which is faster on
-   the workloads measured.  Both give the same frames and counters.  No
+   warps.  The default (0) is the streamed kernel (a lane traces any path of its
+   warp's pixels; bnxSetLaunchConfig and bnxSetScheduling apply to it), which is
+   faster on the workloads measured.  Both give the same frames and counters.  No
    reference counterpart. */
 BN_API void bnxSetRegrouping(BNContext context, int enable);
 /* Warp scheduling of the render kernel: a warp keeps stepping macrocells and
    Woodcock ranges until at least serviceBatch of its lanes (or all of its
    busy lanes) need service -- shading, accumulation, a new ray -- and then
    serves them together (1..32; until it is set, each kernel's own default:
-   22 plain, 12 multi-scatter, 28 isosurface). */
+   22 plain, 12 multi-scatter, 28 isosurface; a value set here, or found by
+   bnxAutotuneBatch, is every kernel's from then on). */
 BN_API void bnxSetScheduling(BNContext context, int serviceBatch);
 /* Bounds-checked build (libbarney_b200_bc.so, python -m barney_b200.build
    --bounds-check): every indexed access of the render and macrocell kernels
@@ -332,9 +335,10 @@ BN_API void bnxSetScheduling(BNContext context, int serviceBatch);
    it), -1 in the normal build, -2 on error. */
 BN_API long long bnxBoundsViolations(BNContext context);
 /* Host-side fault injection for tests: after afterAllocations more device
-   allocations (frame buffers, textures, macrocell grids, server buffers), the
-   next one fails once with error 6 (out of memory), made on the host; no CUDA
-   call fails.  A negative count disables it. */
+   allocations (frame buffers, textures, macrocell grids, server buffers, path
+   rings), the next one fails once with error 6 (out of memory), made on the host;
+   no CUDA call fails.  Path rings that cannot be had are tried at half the size
+   instead.  A negative count disables it. */
 BN_API void bnxInjectAllocationFailure(int afterAllocations);
 
 /* Checkpoint / resume of a frame buffer's progressive state (the reference's

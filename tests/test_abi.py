@@ -69,8 +69,8 @@ def test_kernels_compiled_for_sm100a():
     log = open(os.path.join(ROOT, "barney_b200", "csrc", "ptxas.log")).read()
     assert "for 'sm_100a'" in log
     assert "renderKernel" in log
-    # The plain render kernels are capped at 7 blocks of 128 threads per SM
-    # (72 registers), those that test compensation per job at 6 (80), the
+    # The plain kernels -- streamed, and the lane-owned one of the no-allocation
+    # path -- are capped at 7 blocks of 128 threads per SM (72 registers), the
     # multi-scatter ones at 5 (96) and the isosurface ones (EXT 2 and 3) at 4
     # (128); the spill bytes that costs are a measured trade for the extra
     # blocks.  A large spill would mean a regression.
@@ -84,6 +84,12 @@ def test_kernels_compiled_for_sm100a():
         args = re.findall(r"Li(n?\d+)E", name.split("EEv")[0])
         ext = int(args[2] if "renderKernel" in name.split("I")[0] else args[1])
         assert m and int(m.group(1)) <= 320, (ext, b.splitlines()[1])
+    # streamKernel, streamBatchKernel, streamBatchParamKernel, exact and fast-math
+    streamed = [b for b in blocks[1:] if re.match(r"_ZN3bnb(8fastmath)?\d+stream(Batch|BatchParam)?Kernel", b.split()[0])]
+    assert len(streamed) >= 22 * 2
+    for b in streamed:
+        m = re.search(r"(\d+) bytes spill stores", b)
+        assert m and int(m.group(1)) <= 320, b.splitlines()[:2]
 
 
 def test_header_compiles_as_c_and_shim_as_cpp(tmp_path):

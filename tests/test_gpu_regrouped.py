@@ -1,12 +1,12 @@
 """The regrouped render kernel (bnxSetRegrouping): pixel slots in shared
 memory, taken by warps from ring queues (new pixels, rays to trace,
 collisions to shade, rays that ended).  It must give the
-per-lane kernel's frames and work counters bit for bit (both are checked
+streamed kernel's frames and work counters bit for bit (both are checked
 against the CPU oracle here), over every plain scene of the parity tests,
 accumulation across renders and compensated accumulation, pixel partitions,
 degenerate frame shapes, the fast-math object's instance, and a render
 deadline that aborts the frame and leaves the context usable.  (It is not
-the default: on the workloads measured the per-lane kernel is faster.)"""
+the default: on the workloads measured the streamed kernel is faster.)"""
 import numpy as np
 import pytest
 
@@ -47,7 +47,7 @@ def test_regrouped_accumulation_across_renders(compensated):
     d = small_noise_scene(w=45, h=31, compensated_accum=compensated)
     img, _ = regrouped_render(d, 2, renders=3)
     want, _ = regrouped_render(d, 2, renders=3, regroup=False)
-    assert_bitexact(img, want, "3 x 2 waves, regrouped vs per-lane")
+    assert_bitexact(img, want, "3 x 2 waves, regrouped vs streamed")
     if not compensated:
         ref, _, _ = oracle_render(d, 6)
         assert_bitexact(img, ref, "3 x 2 waves")
@@ -70,7 +70,7 @@ def test_regrouped_partitions_and_fast_math():
     owners = bn.partition_owners(67, 45, 3)
     assert_bitexact(bn.merge_partitions(np.stack(parts), owners), full, "3 partitions")
     # the fast-math object's regrouped kernel runs, close to the fast-math
-    # per-lane kernel (the two are compiled separately, so fused operations
+    # streamed kernel (the two are compiled separately, so fused operations
     # may differ between them)
     df = dict(d, fast_math=True)
     a, sa = regrouped_render(df, 16)
