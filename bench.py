@@ -469,7 +469,7 @@ def run_ours(args):
             "higher_is_better": True, "scaling": "strong" if tile_dp else "weak", "vs_baseline": None,
             "dtype": d["dtype"],
             "data": "synthetic (seeded value noise / Gaussian blobs generated on device)",
-            "config": dict(desc, kernel=args.kernel,
+            "config": dict(desc, kernel="lane-owned" if d.get("max_volume_bounces") or d.get("iso") else args.kernel,
                            parallelism=(f"pixel tiles x{world}, NCCL all-gather per frame" if tile_dp
                                               else f"replicas x{world}" if world > 1 else "single GPU"),
                            l2="inputs larger than L2" if flush is None
